@@ -885,92 +885,204 @@ bool Executor::fused_pays(const Segment& seg) {
 void Executor::run_vm(const Segment& seg) {
   const int n_nodes = static_cast<int>(nodes_.size());
   constexpr int32_t kNone = INT32_MIN;
-  std::vector<int32_t> loc(n_nodes, kNone);
-  std::vector<const uint64_t*> ext;
-  auto ext_of = [&](const uint64_t* p) {
-    ext.push_back(p);
-    return -static_cast<int32_t>(ext.size());
-  };
-  for (int i : seg.inputs) loc[i] = ext_of(nodes_[i].buf ? nodes_[i].buf->p : const_ptr(i));
   std::vector<uint8_t> is_out(n_nodes, 0);
   for (int o : seg.outputs) is_out[o] = 1;
+  // x & ~y with a ~y that nothing else reads is one instruction
+  std::vector<int32_t> uses(n_nodes, 0);
+  for (int id : seg.order)
+    for (int o : {nodes_[id].a, nodes_[id].b})
+      if (o >= 0) ++uses[o];
+  for (int id : seg.outputs) ++uses[id];
+  for (auto& p : seg.pops) ++uses[p.first];
+  struct Op { int a, b; bool and_not; };
+  auto operands = [&](int id) -> Op {
+    const Node& x = nodes_[id];
+    if (x.op == NOp::And) {
+      auto folds = [&](int o) { return nodes_[o].op == NOp::Not && pending(o) && uses[o] == 1; };
+      if (folds(x.b)) return {x.a, nodes_[x.b].a, true};
+      if (folds(x.a)) return {x.b, nodes_[x.a].a, true};
+    }
+    return {x.a, x.b, x.op == NOp::AndNot};
+  };
+  // Depth first from the results, the larger operand first: an instruction
+  // then mostly reads the one before it (from registers), and few values are
+  // live at a time.
+  std::vector<int32_t> size(n_nodes, 0);
+  for (int id : seg.order) {
+    int64_t sz = 1;
+    for (int o : {nodes_[id].a, nodes_[id].b})
+      if (o >= 0) sz += size[o];
+    size[id] = static_cast<int32_t>(std::min<int64_t>(sz, INT32_MAX));
+  }
+  std::vector<int> order;
+  order.reserve(seg.order.size());
+  {
+    std::vector<uint8_t> state(n_nodes, 0);   // 1: operands pushed, 2: placed
+    std::vector<int> stack;
+    auto place = [&](int root) {
+      if (size[root] == 0) return;   // an input
+      stack.push_back(root);
+      while (!stack.empty()) {
+        const int id = stack.back();
+        if (state[id]) {
+          stack.pop_back();
+          if (state[id] == 1) order.push_back(id);
+          state[id] = 2;
+          continue;
+        }
+        state[id] = 1;
+        const Op x = operands(id);
+        int first = x.a, second = x.b;   // pushed last = computed first
+        if (first >= 0 && second >= 0 && size[first] < size[second]) std::swap(first, second);
+        for (int o : {second, first})
+          if (o >= 0 && size[o] > 0 && !state[o]) stack.push_back(o);
+      }
+    };
+    for (int id : seg.outputs) place(id);
+    for (auto& p : seg.pops) place(p.first);
+  }
   std::vector<int64_t> last(n_nodes, -1);
-  for (size_t t = 0; t < seg.order.size(); ++t) {
-    const Node& x = nodes_[seg.order[t]];
+  for (size_t t = 0; t < order.size(); ++t) {
+    const Op x = operands(order[t]);
     if (x.a >= 0) last[x.a] = static_cast<int64_t>(t);
     if (x.b >= 0) last[x.b] = static_cast<int64_t>(t);
   }
-  // popcounts sorted by node (segment order is increasing node id)
+  // popcounts sorted by node
   std::vector<std::pair<int, int64_t>> pops(seg.pops.begin(), seg.pops.end());
   std::stable_sort(pops.begin(), pops.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
+  const int64_t kmax = 64 * nw_;
+
   std::vector<VmOp> ops;
-  ops.reserve(seg.order.size() + pops.size());
-  auto emit_pops = [&](int node) {
-    auto it = std::lower_bound(pops.begin(), pops.end(), std::make_pair(node, int64_t(INT64_MIN)));
-    for (; it != pops.end() && it->first == node; ++it) {
+  std::vector<const uint64_t*> ext;
+  int32_t n_slots = 0;
+  int64_t n_loads = 0;
+  // in_slots: inputs and constants are loaded into slots first, outputs are
+  // computed in slots and stored; else both are reached through the external
+  // table (segments whose inputs do not fit in the value file)
+  auto build = [&](bool in_slots) {
+    ops.clear();
+    ext.clear();
+    n_slots = 0;
+    n_loads = 0;
+    ops.reserve(seg.order.size() + pops.size() + seg.inputs.size() + seg.outputs.size());
+    std::vector<int32_t> loc(n_nodes, kNone);
+    std::vector<int32_t> free_slots;
+    auto ext_of = [&](const uint64_t* p) {
+      ext.push_back(p);
+      return -static_cast<int32_t>(ext.size());
+    };
+    auto new_slot = [&]() {
+      if (free_slots.empty()) return n_slots++;
+      const int32_t v = free_slots.back();
+      free_slots.pop_back();
+      return v;
+    };
+    auto emit_pops = [&](int node) {
+      auto it = std::lower_bound(pops.begin(), pops.end(), std::make_pair(node, int64_t(INT64_MIN)));
+      for (; it != pops.end() && it->first == node; ++it) {
+        VmOp op{};
+        op.code = kVmPop;
+        op.a = loc[node];
+        op.dst = static_cast<int32_t>(it->second);
+        ops.push_back(op);
+      }
+    };
+    auto pointer_hi = [](const uint64_t* p) {
+      return static_cast<int32_t>(static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p) >> 32));
+    };
+    auto pointer_lo = [](const uint64_t* p) {
+      return static_cast<int32_t>(static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p)));
+    };
+    if (in_slots) {
+      for (int i : seg.inputs)
+        if (nodes_[i].buf) {
+          loc[i] = new_slot();
+          VmOp op{};
+          op.code = kVmLoad;
+          op.dst = loc[i];
+          op.a = pointer_lo(nodes_[i].buf->p);
+          op.b = pointer_hi(nodes_[i].buf->p);
+          ops.push_back(op);
+        }
+      n_loads = std::min<int64_t>(static_cast<int64_t>(ops.size()), kVmWindow);
+      for (int i : seg.inputs)
+        if (!nodes_[i].buf) {
+          loc[i] = new_slot();
+          VmOp op{};
+          op.code = kVmFill;
+          op.fill = nodes_[i].op == NOp::Zero ? 0 : nodes_[i].op == NOp::OnesMask ? 1 : 2;
+          op.dst = loc[i];
+          ops.push_back(op);
+        }
+    } else {
+      for (int i : seg.inputs) loc[i] = ext_of(nodes_[i].buf ? nodes_[i].buf->p : const_ptr(i));
+    }
+    for (int i : seg.inputs) emit_pops(i);
+    for (size_t t = 0; t < order.size(); ++t) {
+      const int id = order[t];
+      Node& n = nodes_[id];
+      const Op x = operands(id);
+      if (is_out[id] && !n.buf) n.buf = dev_.alloc_stream(nw_);
+      const int32_t dst = is_out[id] && !in_slots ? ext_of(n.buf->p) : new_slot();
+      loc[id] = dst;
       VmOp op{};
-      op.code = kVmPop;
-      op.a = loc[node];
-      op.dst = static_cast<int32_t>(it->second);
+      op.dst = dst;
+      op.a = loc[x.a];
+      if (x.b >= 0) op.b = loc[x.b];
+      switch (n.op) {
+        case NOp::Not: op.code = kVmNot; break;
+        case NOp::And: op.code = x.and_not ? kVmAndNot : kVmAnd; break;
+        case NOp::Or: op.code = kVmOr; break;
+        case NOp::Xor: op.code = kVmXor; break;
+        case NOp::AndNot: op.code = kVmAndNot; break;
+        case NOp::Add: op.code = kVmAdd; break;
+        case NOp::Shl: op.code = kVmShl; op.b = static_cast<int32_t>(std::min<int64_t>(n.k, kmax)); break;
+        case NOp::Shr:
+          op.code = kVmShr;
+          op.b = static_cast<int32_t>(std::min<int64_t>(n.k, kmax));
+          op.fill = nodes_[n.a].tail ? 1 : 0;
+          break;
+        default: throw RuntimeError("internal: unexpected node in VM segment");
+      }
+      if (op.a == kNone || (x.b >= 0 && op.b == kNone))
+        throw RuntimeError("internal: VM operand has no location");
       ops.push_back(op);
+      if (is_out[id] && in_slots) {
+        VmOp st{};
+        st.code = kVmStore;
+        st.a = dst;
+        st.dst = pointer_lo(n.buf->p);
+        st.b = pointer_hi(n.buf->p);
+        ops.push_back(st);
+      }
+      emit_pops(id);
+      for (int operand : {x.a, x.b}) {
+        if (operand < 0 || loc[operand] < 0 || last[operand] != static_cast<int64_t>(t)) continue;
+        free_slots.push_back(loc[operand]);
+        if (x.a == x.b) break;   // x op x: free once
+      }
+      if (dst >= 0 && last[id] < 0) free_slots.push_back(dst);   // read by its popcounts or its store only
     }
   };
-  for (int i : seg.inputs) emit_pops(i);
-  std::vector<int32_t> free_slots;
-  int32_t n_slots = 0;
-  const int64_t kmax = 64 * nw_;
-  for (size_t t = 0; t < seg.order.size(); ++t) {
-    const int id = seg.order[t];
-    Node& n = nodes_[id];
-    int32_t dst;
-    if (is_out[id]) {
-      n.buf = dev_.alloc_stream(nw_);
-      dst = ext_of(n.buf->p);
-    } else if (!free_slots.empty()) {
-      dst = free_slots.back();
-      free_slots.pop_back();
-    } else {
-      dst = n_slots++;
-    }
-    loc[id] = dst;
-    VmOp op{};
-    op.dst = dst;
-    op.a = loc[n.a];
-    switch (n.op) {
-      case NOp::Not: op.code = kVmNot; break;
-      case NOp::And: op.code = kVmAnd; op.b = loc[n.b]; break;
-      case NOp::Or: op.code = kVmOr; op.b = loc[n.b]; break;
-      case NOp::Xor: op.code = kVmXor; op.b = loc[n.b]; break;
-      case NOp::AndNot: op.code = kVmAndNot; op.b = loc[n.b]; break;
-      case NOp::Add: op.code = kVmAdd; op.b = loc[n.b]; break;
-      case NOp::Shl: op.code = kVmShl; op.b = static_cast<int32_t>(std::min<int64_t>(n.k, kmax)); break;
-      case NOp::Shr:
-        op.code = kVmShr;
-        op.b = static_cast<int32_t>(std::min<int64_t>(n.k, kmax));
-        op.fill = nodes_[n.a].tail ? 1 : 0;
-        break;
-      default: throw RuntimeError("internal: unexpected node in VM segment");
-    }
-    if (op.a == kNone || ((n.op == NOp::And || n.op == NOp::Or || n.op == NOp::Xor || n.op == NOp::AndNot ||
-                           n.op == NOp::Add) && op.b == kNone))
-      throw RuntimeError("internal: VM operand has no location");
-    ops.push_back(op);
-    emit_pops(id);
-    for (int operand : {n.a, n.b}) {
-      if (operand < 0 || loc[operand] < 0 || last[operand] != static_cast<int64_t>(t)) continue;
-      if (operand == n.b && n.a == n.b) continue;   // x op x: free once
-      free_slots.push_back(loc[operand]);
-    }
-    if (!is_out[id] && last[id] < 0) free_slots.push_back(dst);   // computed only for its popcounts
+  VmPlan plan;
+  bool in_slots = vm_plan(1, nw_, 0).ctas > 0;
+  if (in_slots) {
+    build(true);
+    plan = vm_plan(n_slots, nw_, 0);
+    // inputs read in place leave room for the file in shared memory
+    if (!plan.smem) in_slots = false;
+  }
+  if (!in_slots) {
+    build(false);
+    plan = vm_plan(n_slots, nw_, 0);
   }
   if (ops.empty()) return;
+  if (plan.ctas > 0) vm_finish(ops, n_slots, static_cast<int64_t>(ext.size()), n_loads, plan);
   // device copies: instruction list | pointer table | slot file (if global)
   auto align = [](size_t b) { return (b + 255) & ~size_t(255); };
   const size_t ops_b = ops.size() * sizeof(VmOp);
   const size_t ext_b = std::max<size_t>(1, ext.size()) * sizeof(uint64_t*);
-  const bool smem = vm_smem_bytes(n_slots, nw_) > 0;
-  const size_t file_b = smem ? 0 : static_cast<size_t>(n_slots) * static_cast<size_t>(nw_) * 8;
-  const size_t total = align(ops_b) + align(ext_b) + file_b;
+  const size_t total = align(ops_b) + align(ext_b) + static_cast<size_t>(plan.file_words) * 8;
   if (total > vm_cap_) {
     // the old block returns to the device cache; stream order keeps it
     // alive for work already queued on it
@@ -981,13 +1093,14 @@ void Executor::run_vm(const Segment& seg) {
   char* base = static_cast<char*>(vm_buf_);
   VmOp* d_ops = reinterpret_cast<VmOp*>(base);
   const uint64_t** d_ext = reinterpret_cast<const uint64_t**>(base + align(ops_b));
-  uint64_t* d_file = smem ? nullptr : reinterpret_cast<uint64_t*>(base + align(ops_b) + align(ext_b));
+  uint64_t* d_file =
+      plan.smem || plan.file_words == 0 ? nullptr : reinterpret_cast<uint64_t*>(base + align(ops_b) + align(ext_b));
   BSZ_CUDA(cudaMemcpyAsync(d_ops, ops.data(), ops_b, cudaMemcpyHostToDevice, dev_.stream()));
   if (!ext.empty())
     BSZ_CUDA(cudaMemcpyAsync(d_ext, ext.data(), ext.size() * sizeof(uint64_t*), cudaMemcpyHostToDevice,
                              dev_.stream()));
-  VmLaunch L{d_ops, static_cast<int64_t>(ops.size()), d_ext, d_file, n_slots, nw_, last_mask_, d_slots_};
-  launch_vm(dev_, L);
+  VmLaunch L{d_ops, static_cast<int64_t>(ops.size()), n_loads, ext.empty() ? nullptr : d_ext, d_file, n_slots, nw_, last_mask_, d_slots_};
+  launch_vm(dev_, L, plan);
   ++vm_launches;
   max_live_buffers = std::max(max_live_buffers, live_buffer_count() + n_slots);
 }

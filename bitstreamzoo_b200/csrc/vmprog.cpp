@@ -1,6 +1,7 @@
 // Whole programs on the device interpreter: the AST, control flow included,
-// compiled to one instruction list that a single CTA runs (vm.cu, program
-// mode).  An if/while condition is a CTA-wide OR on the device, so a program
+// compiled to one instruction list that one launch of the device interpreter
+// runs (vm.cu, program mode).  An if/while condition is an OR over its
+// threads on the device, so a program
 // such as a multi-pattern regex matcher (thousands of `if` guards, a while
 // loop per MatchStar fixpoint) costs one launch and one read-back instead of
 // one host round trip per condition.
@@ -11,7 +12,7 @@
 // the branches need no merge), for-loops unroll with host-known bounds,
 // ints known on the host stay constants, and ints that depend on a popcount
 // or on a branch live in device registers.  Tails are device state because a
-// branch can change them.  Op counts are counted on the device per class.
+// branch can change them.  Op counts follow from each region's entry count.
 //
 // A program runs here only if nothing in it needs the host mid-run: a device
 // int used as a loop bound, array index, array size or shift amount; an
@@ -34,15 +35,19 @@ namespace bsz {
 namespace {
 struct NotEligible {};
 constexpr int32_t kSlotZero = 0, kSlotMask = 1, kSlotAll = 2, kSlotTmp = 3, kFixedSlots = 4;
+// Op-count classes; kClsNone = not counted.
+enum OpClass : uint8_t {
+  kClsNone = 0, kClsNot, kClsAnd, kClsOr, kClsXor, kClsAdd, kClsShl, kClsShr, kClsPop, kClsCount
+};
 }  // namespace
 
 struct VmCompiler {
   Executor& ex;
   const Program& prog;
   std::vector<VmOp> code;
-  std::vector<const uint64_t*> ext;
   int32_t n_slots = kFixedSlots;
   int32_t n_iregs = 0;
+  int64_t n_loads = 0;
   int depth = 0;
   int32_t zero_reg = -1;
 
@@ -71,6 +76,28 @@ struct VmCompiler {
   // defined before it
   std::vector<std::vector<int>> region_streams, region_ints;
 
+  // Counted operations of every region (the program's top level, each
+  // conditional body) and the int register that counts its entries (-1: once):
+  // the instructions of a region all run each time it is entered.
+  struct Region {
+    int32_t entries = -1;
+    int64_t ops[kClsCount] = {};
+  };
+  std::vector<Region> regions{Region{}};
+  std::vector<size_t> open_regions{0};
+  void open_body() {   // at the first instruction of a conditional body
+    const int32_t r = new_ireg();
+    open_regions.push_back(regions.size());
+    regions.push_back(Region{});
+    regions.back().entries = r;
+    op(kVmInc, r);
+    ++depth;
+  }
+  void close_body() {
+    --depth;
+    open_regions.pop_back();
+  }
+
   explicit VmCompiler(Executor& e) : ex(e), prog(e.prog_) {
     const size_t nn = prog.names.size();
     slot_of.assign(nn, -1);
@@ -86,15 +113,17 @@ struct VmCompiler {
     o.dst = dst;
     o.a = a;
     o.b = b;
-    o.cls = cls;
     o.fill = fill;
     code.push_back(o);
+    ++regions[open_regions.back()].ops[cls];
   }
   int32_t new_slot() { return n_slots++; }
   int32_t new_ireg() { return n_iregs++; }
-  int32_t ext_of(const uint64_t* p) {
-    ext.push_back(p);
-    return static_cast<int32_t>(ext.size() - 1);
+  static int32_t pointer_lo(const uint64_t* p) {
+    return static_cast<int32_t>(static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p)));
+  }
+  static int32_t pointer_hi(const uint64_t* p) {
+    return static_cast<int32_t>(static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p) >> 32));
   }
   void iconst(int32_t reg, int64_t v) {
     const uint64_t u = static_cast<uint64_t>(v);
@@ -109,7 +138,9 @@ struct VmCompiler {
       case NOp::Zero: op(kVmCopy, slot, kSlotZero); break;
       case NOp::OnesMask: op(kVmCopy, slot, kSlotMask); break;
       case NOp::AllOnes: op(kVmCopy, slot, kSlotAll); break;
-      case NOp::Buf: op(kVmLoad, slot, ext_of(n.buf->p), 0, kClsNone, n.tail); break;
+      case NOp::Buf:
+        op(kVmLoad, slot, pointer_lo(n.buf->p), pointer_hi(n.buf->p), kClsNone, n.tail);
+        break;
       default: throw NotEligible{};   // a pending computation: not a fresh run
     }
   }
@@ -144,6 +175,11 @@ struct VmCompiler {
         ints[id].v = ex.ints_[id].v;
       }
     }
+    // loads first (each slot is set once here, so their order is free): the
+    // device issues them all before the first instruction
+    n_loads = std::stable_partition(code.begin(), code.end(), [](const VmOp& o) { return o.code == kVmLoad; }) -
+              code.begin();
+    n_loads = std::min<int64_t>(n_loads, kVmWindow);
   }
 
   // ---- definedness
@@ -382,9 +418,9 @@ struct VmCompiler {
         prescan(s.body);
         const size_t jz = code.size();
         op(kVmJz, 0, c, 0);
-        ++depth;
+        open_body();
         stmts(s.body);
-        --depth;
+        close_body();
         leave_region();
         code[jz].b = static_cast<int32_t>(code.size());
         return;
@@ -399,9 +435,9 @@ struct VmCompiler {
         const size_t jz = code.size();
         op(kVmJz, 0, c, 0);
         op(kVmTick, ctr);
-        ++depth;
+        open_body();
         stmts(s.body);
-        --depth;
+        close_body();
         leave_region();
         op(kVmJmp, 0, 0, top);
         code[jz].b = static_cast<int32_t>(code.size());
@@ -462,17 +498,17 @@ bool Executor::run_vm_program() {
     if (c.ints[id].def && c.int_cond_only[id]) return false;
   for (auto& o : outs) {
     o.buf = dev_.alloc_stream(nw_);
-    c.op(kVmStore, c.ext_of(o.buf->p), o.slot);
+    c.op(kVmStore, VmCompiler::pointer_lo(o.buf->p), o.slot, VmCompiler::pointer_hi(o.buf->p));
   }
 
-  // device buffers: instructions | pointer table | state | slot file (if global)
+  // device buffers: instructions | state | slot file (if global)
   auto align = [](size_t b) { return (b + 255) & ~size_t(255); };
+  const VmPlan plan = vm_plan(c.n_slots, nw_, vm_prog_warp_bytes(c.n_iregs, c.n_slots));
+  vm_mark_tails(c.code, c.n_slots);
+  if (plan.ctas > 0) vm_finish(c.code, c.n_slots, 0, c.n_loads, plan);
   const size_t ops_b = c.code.size() * sizeof(VmOp);
-  const size_t ext_b = std::max<size_t>(1, c.ext.size()) * sizeof(uint64_t*);
   const size_t state_b = vm_state_bytes(c.n_iregs, c.n_slots);
-  const bool smem = vm_smem_bytes(c.n_slots, nw_) > 0;
-  const size_t file_b = smem ? 0 : static_cast<size_t>(c.n_slots) * static_cast<size_t>(nw_) * 8;
-  const size_t total = align(ops_b) + align(ext_b) + align(state_b) + file_b;
+  const size_t total = align(ops_b) + align(state_b) + static_cast<size_t>(plan.file_words) * 8;
   if (total > vm_cap_) {
     // the old block returns to the device cache; stream order keeps it
     // alive for work already queued on it
@@ -482,18 +518,14 @@ bool Executor::run_vm_program() {
   }
   char* base = static_cast<char*>(vm_buf_);
   VmOp* d_ops = reinterpret_cast<VmOp*>(base);
-  const uint64_t** d_ext = reinterpret_cast<const uint64_t**>(base + align(ops_b));
-  uint8_t* d_state = reinterpret_cast<uint8_t*>(base + align(ops_b) + align(ext_b));
+  uint8_t* d_state = reinterpret_cast<uint8_t*>(base + align(ops_b));
   uint64_t* d_file =
-      smem ? nullptr : reinterpret_cast<uint64_t*>(base + align(ops_b) + align(ext_b) + align(state_b));
+      plan.file_words == 0 ? nullptr : reinterpret_cast<uint64_t*>(base + align(ops_b) + align(state_b));
   dev_.h2d(d_ops, c.code.data(), ops_b);
-  if (!c.ext.empty())
-    BSZ_CUDA(cudaMemcpyAsync(d_ext, c.ext.data(), c.ext.size() * sizeof(uint64_t*), cudaMemcpyHostToDevice,
-                             dev_.stream()));
-  BSZ_CUDA(cudaMemsetAsync(d_state, 0, state_b, dev_.stream()));
-  VmProgLaunch L{{d_ops, static_cast<int64_t>(c.code.size()), d_ext, d_file, c.n_slots, nw_, last_mask_, nullptr},
+  VmProgLaunch L{{d_ops, static_cast<int64_t>(c.code.size()), c.n_loads, nullptr, d_file, c.n_slots, nw_, last_mask_,
+                  nullptr},
                  d_state, c.n_iregs};
-  launch_vm_program(dev_, L);
+  launch_vm_program(dev_, L, plan);
   ++vm_launches;
   ++n_segments;
   std::vector<uint8_t> st(state_b);
@@ -508,20 +540,22 @@ bool Executor::run_vm_program() {
   if (err == kVmErrNegShift) throw RuntimeError("negative shift count");
   if (err) throw RuntimeError("device interpreter error " + std::to_string(err));
   static const char* const kNames[kClsCount] = {"", "~", "&", "|", "^", "+", "<<", ">>", "popcount"};
-  for (int k = 1; k < kClsCount; ++k) {
-    uint64_t n = 0;
-    std::memcpy(&n, st.data() + 8 + 8 * k, 8);
-    if (n) {
-      op_count += static_cast<int64_t>(n);
-      op_mix[kNames[k]] += static_cast<int64_t>(n);
-    }
-  }
-  const uint8_t* tails = st.data() + 8 + 8 * kClsCount + 8 * static_cast<size_t>(c.n_iregs);
+  const uint8_t* tails = st.data() + 8 + 8 * static_cast<size_t>(c.n_iregs);
   auto ireg = [&](int32_t r) {
     int64_t v = 0;
-    std::memcpy(&v, st.data() + 8 + 8 * kClsCount + 8 * static_cast<size_t>(r), 8);
+    std::memcpy(&v, st.data() + 8 + 8 * static_cast<size_t>(r), 8);
     return v;
   };
+  for (const auto& region : c.regions) {
+    const int64_t entries = region.entries < 0 ? 1 : ireg(region.entries);
+    for (int k = 1; k < kClsCount; ++k) {
+      const int64_t n = entries * region.ops[k];
+      if (n) {
+        op_count += n;
+        op_mix[kNames[k]] += n;
+      }
+    }
+  }
   // results into the executor's state, as its own walk would leave them
   for (auto& o : outs) {
     const int node = buf_node(o.buf, tails[o.slot], false);
