@@ -13,10 +13,10 @@
 //      - shifts of an input read the neighbouring words from memory.
 //  * A warp's first step needs the state at the start of its range.  It is
 //    obtained by speculation: the warp first processes H warm-up words before
-//    its range from an all-zero state while tracking, per node, how far the
-//    possibly-wrong ("dirty") prefix reaches (additions stop being dirty at
-//    the first word whose sum is not all ones; shifts move the dirt by their
-//    distance).  If the dirt has died out before the range starts the state
+//    its range from an all-zero state while tracking, per node and in bits,
+//    how far the possibly-wrong ("dirty") prefix reaches (an addition is clean
+//    above the first clean bit where its operands are equal, which decides the
+//    carry; shifts move the dirt by their distance).  If the dirt has died out before the range starts the state
 //    is exact; otherwise the warm-up is doubled (up to 8 times).  If it still
 //    cannot be proven exact the kernel raises a flag and the host re-runs the
 //    segment with the plain per-op kernels, which are exact by construction.
@@ -150,6 +150,15 @@ struct Part {
                                               // the plain carry-scan kernel (decoupled look-back)
 };
 
+// Bits that an addition's carry is taken to need until it is decided (where
+// the operands' bits are equal), for the length of the first warm-up; what
+// really happens is tracked on the device.
+constexpr int64_t kAddSettle = 4;
+
+// One kernel of the warp form.  Dirt is tracked in bits, not words: a chain of 40 one-bit shifts and 20
+// additions dirties about 120 bits, which 4 warm-up words settle; counted as
+// one word per operation it took 64 words and four doublings (a 200-op DAG of
+// 2^26 bits, thread form, on a B200: 61 us, 34 us with bits).
 struct Gen {
   const std::vector<Node>& nodes;
   const Part& part;
@@ -167,7 +176,7 @@ struct Gen {
   std::vector<std::pair<int, int>> outs;   // (node, output index); a node may repeat
   std::set<int> in_part;           // computed in this part
   std::set<int> shl_src;           // temporaries shifted left (need previous-step value)
-  std::map<int, int> shl_ws;       // max word shift per shl source temporary
+  std::map<int, int64_t> shl_k;    // max shift (bits) per shl source temporary
   // Shifted temporaries whose every left shift is by 1 or 2 bits: the bits
   // shifted in come from the top bits of the word below, which one ballot
   // per bit delivers to every lane; across steps only those 1-2 bits of the
@@ -188,8 +197,8 @@ struct Gen {
   std::map<int, int> last_small_use;
   std::string pk(int bitpos) const { return "pk" + std::to_string(bitpos / 32); }
   std::vector<uint8_t> dyn;        // node dirt must be tracked during warm-up
-  std::map<int, int64_t> sdh;      // static dirt (words) for nodes without add ancestors
-  int64_t warm = 64;               // warm-up words
+  std::map<int, int64_t> sdh;      // static dirt (bits) for nodes without add ancestors
+  int64_t warm = 32;               // warm-up words
   // Global loads of one step ("load slots"): expression templates over @W@
   // (this lane's word) and @B@ (the step's first word), de-duplicated.  The
   // owned-range loop issues them one step ahead of the arithmetic.
@@ -258,17 +267,19 @@ struct Gen {
       for (size_t i = 0; i < part.outputs.size(); ++i) outs.push_back({part.outputs[i], static_cast<int>(i)});
     for (int n : part.order) in_part.insert(n);
     dyn.assign(nodes.size(), 0);
-    int64_t max_static = 0;
+    int64_t max_dirt = 0;
+    std::map<int, int64_t> likely;   // dirt (bits), additions taken to settle in kAddSettle
     for (int n : part.order) {
       const Node& x = nodes[n];
-      auto d = [&](int o) -> int64_t { return (o >= 0 && sdh.count(o)) ? sdh[o] : 0; };
-      bool dy = false;
+      auto d = [&](const std::map<int, int64_t>& m, int o) -> int64_t {
+        auto it = m.find(o);
+        return it == m.end() ? 0 : it->second;
+      };
+      bool dy = x.op == NOp::Add;
       for (int o : {x.a, x.b})
         if (o >= 0 && dyn[o]) dy = true;
-      int64_t s = std::max(d(x.a), d(x.b));
-      if (x.op == NOp::Add) dy = true;
+      int64_t shift = 0;
       if (x.op == NOp::Shl && x.a >= 0 && in_part.count(x.a)) {
-        int ws = static_cast<int>(x.k / 64);
         const bool small = x.k >= 1 && x.k <= 2;
         if (!shl_src.count(x.a)) {
           if (small) small_shl[x.a] = static_cast<int>(x.k);
@@ -277,17 +288,15 @@ struct Gen {
           else small_shl.erase(x.a);
         }
         shl_src.insert(x.a);
-        shl_ws[x.a] = std::max(shl_ws[x.a], ws);
-        s = d(x.a) + ws + ((x.k % 64) ? 1 : 0);
+        shl_k[x.a] = std::max(shl_k[x.a], x.k);
+        shift = x.k;
       }
       dyn[n] = dy;
-      if (!dy) {
-        sdh[n] = s;
-        max_static = std::max(max_static, s);
-      }
+      if (!dy) sdh[n] = std::max(d(sdh, x.a), d(sdh, x.b)) + shift;
+      likely[n] = std::max(d(likely, x.a), d(likely, x.b)) + shift + (x.op == NOp::Add ? kAddSettle : 0);
+      max_dirt = std::max(max_dirt, likely[n]);
     }
-    warm = ((max_static + 64 + 31) / 32) * 32;
-    if (warm > 8192) warm = 8192;
+    warm = std::min<int64_t>(8192, ((max_dirt + 63) / 64 + 1 + 31) / 32 * 32);
     int nb = 0;
     for (int n : part.order)
       if (nodes[n].op == NOp::Add) cbit[n] = nb++;
@@ -398,11 +407,19 @@ struct Gen {
             << "        const u32 G = __ballot_sync(~0u, sa < " << a << ");\n"
             << "        const u32 P = __ballot_sync(~0u, sa == ~0ull);\n";
           if (track && dyn[n]) {
+            // the first bit at or past the operands' dirt where they are equal
             s << "        if (!res" << n << ") {\n"
-              << "          const int d0 = max(" << dh(x.a) << ", " << dh(x.b) << ") - rel;\n"
-              << "          if (d0 < 32) {\n"
-              << "            const u32 cand = ~P & (d0 <= 0 ? ~0u : (~0u << d0));\n"
-              << "            if (cand) { res" << n << " = 1; dh" << n << " = rel + __ffs(cand); }\n"
+              << "          const int d0 = max(" << dh(x.a) << ", " << dh(x.b) << ") - 64 * rel;\n"
+              << "          if (d0 < 2048) {\n"
+              << "            const int l0 = d0 > 0 ? d0 >> 6 : 0;\n"
+              << "            u64 np = lane < l0 ? 0ull : ~(" << a << " ^ " << b << ");\n"
+              << "            if (lane == l0 && d0 > 0) np &= ~0ull << (d0 & 63);\n"
+              << "            const u32 hit = __ballot_sync(~0u, np != 0ull);\n"
+              << "            if (hit) {\n"
+              << "              const int f = __ffs(hit) - 1;\n"
+              << "              res" << n << " = 1;\n"
+              << "              dh" << n << " = 64 * (rel + f) + __shfl_sync(~0u, __ffsll((long long)np), f);\n"
+              << "            }\n"
               << "          }\n"
               << "        }\n";
           }
@@ -505,9 +522,7 @@ struct Gen {
         s << "      " << v(n) << " &= lm;\n";
       if (track && dyn[n] && x.op != NOp::Add) {
         if (x.op == NOp::Shl && in_part.count(x.a) && !is_input(x.a)) {
-          int64_t ws = x.k / 64;
-          int bs = static_cast<int>(x.k % 64);
-          s << "      dh" << n << " = min(" << dh(x.a) << " + " << (ws + (bs ? 1 : 0)) << ", 1 << 30);\n";
+          s << "      dh" << n << " = min(" << dh(x.a) << " + " << x.k << ", 1 << 30);\n";
         } else {
           s << "      dh" << n << " = max(" << dh(x.a) << ", " << dh(x.b) << ");\n";
         }
@@ -528,7 +543,7 @@ struct Gen {
     }
   }
 
-  // dirt expression for operand o during warm-up tracking
+  // dirt (bits) expression for operand o during warm-up tracking
   std::string dh(int o) const {
     if (o < 0) return "0";
     if (!in_part.count(o)) return "0";   // inputs / constants are exact
@@ -602,14 +617,15 @@ struct Gen {
       s << "    for (long long base = p0; base < s; base += 32) {\n";
       emit_step(s, true, false);
       s << "    }\n";
-      // exactness: every carry and every previous-step value at s is exact
-      s << "    const int need = (int)(s - p0);\n    bool ok = true;\n";
+      // exactness: every carry into s, and the bits below s that a shift
+      // brings into the range, are exact
+      s << "    const int need = 64 * (int)(s - p0);\n    bool ok = true;\n";
       for (int n : adds)
         if (dyn[n]) s << "    ok = ok && res" << n << " && dh" << n << " <= need;\n";
       for (int n : shl_src) {
-        if (dyn[n]) s << "    ok = ok && dh" << n << " <= need - 32;\n";
+        if (dyn[n]) s << "    ok = ok && dh" << n << " <= need - " << shl_k.at(n) << ";\n";
         else if (sdh.count(n) && sdh.at(n) > 0)
-          s << "    ok = ok && " << sdh.at(n) << " <= need - 32;\n";
+          s << "    ok = ok && " << sdh.at(n) << " <= need - " << shl_k.at(n) << ";\n";
       }
       s << "    if (ok || p0 == 0) break;\n"
         << "    if (attempt >= 8) { if (lane == 0) atomicOr(A.fail, 1u); break; }\n"
@@ -660,9 +676,8 @@ struct Gen {
 // (and any chunk whose shifted loads would leave [0, nw)) take a scalar path
 // with bounds, tail fill and last-word masking.  The state at the start of a
 // thread's range comes from speculation as in the warp form: H warm-up words
-// from an all-zero state, per-node dirt tracking (an addition is exact after
-// the first word where a ^ b is not all ones, at or after its operands' dirt),
-// doubled up to 8 times, then the fail flag and the exact per-op fallback.
+// from an all-zero state, per-node dirt tracking in bits, doubled up to 8
+// times, then the fail flag and the exact per-op fallback.
 struct GenSeq {
   const std::vector<Node>& nodes;
   const Part& part;
@@ -675,7 +690,8 @@ struct GenSeq {
   std::set<int> in_part;
   std::set<int> prev_src;            // nodes whose previous word a shift (k < 64) reads
   std::vector<uint8_t> dyn;
-  std::map<int, int64_t> sdh;        // static dirt (words) of nodes without add ancestors
+  std::map<int, int64_t> sdh;        // static dirt (bits) of nodes without add ancestors
+  std::map<int, int64_t> prev_k;     // max shift (bits) of the nodes in prev_src
   int64_t warm = 4;                  // warm-up words (multiple of 4)
   std::vector<int> emit_order;
   // shifted input reads by a word offset: (node, word offset) -> slot; the
@@ -719,28 +735,35 @@ struct GenSeq {
       for (size_t i = 0; i < part.outputs.size(); ++i) outs.push_back({part.outputs[i], static_cast<int>(i)});
     for (int n : part.order) in_part.insert(n);
     dyn.assign(nodes.size(), 0);
-    // Static dirt of nodes without an addition among their ancestors, in
-    // BITS: a value exact from bit B shifted left by k < 64 is exact from bit
-    // B + k (sdh keeps the word form, ceil(B / 64), which the warm-up checks
-    // and the run-time tracking of the other nodes use).
-    std::map<int, int64_t> sbits;
-    int64_t max_static_bits = 0;
+    // Dirt in bits: a value exact from bit B shifted left by k < 64 is exact
+    // from bit B + k.
+    std::map<int, int64_t> likely;   // as in the warp form
+    int64_t max_dirt = 0;
     for (int n : part.order) {
       const Node& x = nodes[n];
-      auto d = [&](int o) -> int64_t { return (o >= 0 && sbits.count(o)) ? sbits[o] : 0; };
+      auto d = [&](const std::map<int, int64_t>& m, int o) -> int64_t {
+        auto it = m.find(o);
+        return it == m.end() ? 0 : it->second;
+      };
       bool dy = x.op == NOp::Add;
       for (int o : {x.a, x.b})
         if (o >= 0 && dyn[o]) dy = true;
-      int64_t s = std::max(d(x.a), d(x.b));
+      int64_t shift = 0;
       if (x.op == NOp::Shl) {
         const int64_t ws = x.k / 64;
         if (in_part.count(x.a)) {
           if (ws > 0) throw RuntimeError("fused: shift of a temporary by 64 bits or more in a sequential part");
-          if (x.k > 0) { prev_src.insert(x.a); s = d(x.a) + x.k; }
+          if (x.k > 0) {
+            prev_src.insert(x.a);
+            shift = x.k;
+          }
         } else if (!is_const(nodes[x.a].op)) {
           if (ws == 0) {
             // the previous word of an input is zero at the first warm-up word
-            if (x.k > 0) { prev_src.insert(x.a); s = x.k; }
+            if (x.k > 0) {
+              prev_src.insert(x.a);
+              shift = x.k;
+            }
           } else {
             off_slot[{x.a, -ws}] = 0;
             if (x.k % 64) off_slot[{x.a, -ws - 1}] = 0;
@@ -751,14 +774,13 @@ struct GenSeq {
         off_slot[{x.a, ws}] = 0;
         if (x.k % 64) off_slot[{x.a, ws + 1}] = 0;
       }
+      if (shift) prev_k[x.a] = std::max(prev_k[x.a], shift);
       dyn[n] = dy;
-      if (!dy) {
-        sbits[n] = s;
-        sdh[n] = (s + 63) / 64;
-        max_static_bits = std::max(max_static_bits, s);
-      }
+      if (!dy) sdh[n] = std::max(d(sdh, x.a), d(sdh, x.b)) + shift;
+      likely[n] = std::max(d(likely, x.a), d(likely, x.b)) + shift + (x.op == NOp::Add ? kAddSettle : 0);
+      max_dirt = std::max(max_dirt, likely[n]);
     }
-    warm = std::max<int64_t>(4, (((max_static_bits + 63) / 64 + 2 + 3) / 4) * 4);
+    warm = ((max_dirt + 63) / 64 + 1 + 3) / 4 * 4;
     int k = 0;
     for (auto& kv : off_slot) {
       kv.second = k++;
@@ -878,9 +900,11 @@ struct GenSeq {
           s << "      const u64 " << v(n) << " = " << a << " & ~" << b << (mask_here ? " & lm" : "") << ";\n";
           break;
         case NOp::Add:
-          if (mode == 't' && dyn[n])
-            s << "      if (!res" << n << " && r >= max(" << dh(x.a) << ", " << dh(x.b) << ") && (" << a << " ^ " << b
-              << ") != ~0ull) { res" << n << " = 1; dh" << n << " = r + 1; }\n";
+          if (mode == 't' && dyn[n])   // the first bit at or past the operands' dirt where they are equal
+            s << "      if (!res" << n << ") {\n        const int d0 = max(" << dh(x.a) << ", " << dh(x.b)
+              << ") - 64 * r;\n        if (d0 < 64) {\n          const u64 np = ~(" << a << " ^ " << b
+              << ") & (d0 > 0 ? ~0ull << d0 : ~0ull);\n          if (np) { res" << n << " = 1; dh" << n
+              << " = 64 * r + __ffsll((long long)np); }\n        }\n      }\n";
           s << "      const u64 " << v(n) << " = addc(" << a << ", " << b << ", cy" << n << ")"
             << (mask_here ? " & lm" : "") << ";\n";
           break;
@@ -926,7 +950,7 @@ struct GenSeq {
       }
       if (mode == 't' && dyn[n] && x.op != NOp::Add) {
         if (x.op == NOp::Shl && in_part.count(x.a) && x.k > 0)
-          s << "      dh" << n << " = min(" << dh(x.a) << " + 1, 1 << 30);\n";
+          s << "      dh" << n << " = min(" << dh(x.a) << " + " << x.k << ", 1 << 30);\n";
         else
           s << "      dh" << n << " = max(" << dh(x.a) << ", " << dh(x.b) << ");\n";
       }
@@ -1219,13 +1243,14 @@ struct GenSeq {
         if (dyn[n] && nodes[n].op != NOp::Add) s << "    int dh" << n << " = 0;\n";
       s << "    for (long long w = p0; w < s; ++w) {\n      const int r = (int)(w - p0);\n";
       emit_word(s, 't', 0);
-      s << "    }\n    const int need = (int)(s - p0);\n    bool ok = true;\n";
+      s << "    }\n    const int need = 64 * (int)(s - p0);\n    bool ok = true;\n";
       for (int n : adds)
         if (dyn[n]) s << "    ok = ok && res" << n << " && dh" << n << " <= need;\n";
       for (int n : prev_src) {
         if (!in_part.count(n)) continue;
-        if (dyn[n]) s << "    ok = ok && dh" << n << " <= need - 1;\n";
-        else if (sdh.count(n) && sdh.at(n) > 0) s << "    ok = ok && " << sdh.at(n) << " <= need - 1;\n";
+        if (dyn[n]) s << "    ok = ok && dh" << n << " <= need - " << prev_k.at(n) << ";\n";
+        else if (sdh.count(n) && sdh.at(n) > 0)
+          s << "    ok = ok && " << sdh.at(n) << " <= need - " << prev_k.at(n) << ";\n";
       }
       s << "    if (ok || p0 == 0) break;\n"
         << "    if (attempt >= 8) { atomicOr(A.fail, 1u); break; }\n"
@@ -1680,6 +1705,21 @@ PartKernel part_kernel(const std::vector<Node>& nodes, const Part& p, int64_t N,
 
 }  // namespace
 
+// Units (words or 32-word steps) of a stream that one walker (a thread or a
+// warp) takes.  `resident` walkers fit on the device at once, `full` of them
+// keep its issue slots busy.  A stream long enough gives every resident walker
+// one range of at least `least` units (several warm-ups, which are recomputed
+// work).  A shorter one would leave most of the device idle at that length
+// while each walker's chain of steps sets the time, so its ranges shrink until
+// `full` walkers run: measured on a B200, a 200-op DAG of 2^23 bits takes
+// 79 us (warp form) and 84 us (thread form) in ranges of 64 steps or words and
+// 23 and 16 us in these.
+int64_t range_units(int64_t units, int64_t least, int64_t resident, int64_t full) {
+  auto per = [&](int64_t walkers) { return (units + walkers - 1) / std::max<int64_t>(1, walkers); };
+  return std::max<int64_t>({int64_t(1), per(resident), std::min(least, per(std::min(full, resident)))});
+}
+constexpr int kFullWarps = 12;   // warps per SM that keep the issue slots busy (stall counters: 3.2 per scheduler)
+
 // A launched segment whose speculation flags have not been read yet: its
 // parts, a copy of every node they compute or read (with the buffers, so
 // none returns to the cache while a re-run may need it) and where its
@@ -1881,9 +1921,8 @@ void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
       const int R = pk.roww;
       const int per = sc.ctas_per_sm > 0 ? std::min(sc.ctas_per_sm, pk.tma_blocks_per_sm) : pk.tma_blocks_per_sm;
       const int64_t threads_cap = static_cast<int64_t>(dev.sm_count()) * per * sc.warps * 32;
-      const int64_t min_range = std::max<int64_t>(64, 16 * pk.warm);
-      int64_t threads = std::max<int64_t>(1, std::min(threads_cap, (nw + min_range - 1) / min_range));
-      range = ((nw + threads - 1) / threads + R - 1) / R * R;
+      const int64_t full = static_cast<int64_t>(dev.sm_count()) * kFullWarps * 32;
+      range = (range_units(nw, std::max<int64_t>(64, 16 * pk.warm), threads_cap, full) + R - 1) / R * R;
       range = std::min<int64_t>(std::max<int64_t>(range, R), int64_t(1) << 25);
       const int64_t total = (nw + range - 1) / range;
       blocks = static_cast<int>((total + sc.warps * 32 - 1) / (sc.warps * 32));
@@ -1919,28 +1958,32 @@ void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
       tail[ni + no + 5] = static_cast<uint64_t>(nfull);
       tail[ni + no + 6] = 1;
     } else if (sc.layout >= 1) {
-      // thread-sequential: one range of whole 4-word chunks per thread, at
-      // least 16 warm-ups long; a persistent grid of what stays resident
+      // thread-sequential: one range of whole register chunks per thread, 16
+      // warm-ups long where the stream has that many; a persistent grid of
+      // what stays resident
       const int64_t threads_cap = sc.ctas_per_sm < 0 ? std::numeric_limits<int64_t>::max() / 2
                                                      : static_cast<int64_t>(dev.sm_count()) * per_sm * sc.warps * 32;
-      const int64_t min_range = std::max<int64_t>(64, 16 * pk.warm);
-      int64_t threads = std::max<int64_t>(1, std::min(threads_cap, (nw + min_range - 1) / min_range));
+      const int64_t least = std::max<int64_t>(64, 16 * pk.warm);
       const int64_t cw = sc.chunk_words == 8 ? 8 : 4;
-      range = ((nw + threads - 1) / threads + cw - 1) / cw * cw;
+      const int64_t full = sc.ctas_per_sm < 0 ? 0 : static_cast<int64_t>(dev.sm_count()) * kFullWarps * 32;
+      range = full ? range_units(nw, least, threads_cap, full) : least;
+      range = (range + cw - 1) / cw * cw;
       range = std::min<int64_t>(std::max<int64_t>(range, cw), int64_t(1) << 25);   // per-thread popcounts fit u32
       const int64_t total = (nw + range - 1) / range;
       blocks = static_cast<int>((total + sc.warps * 32 - 1) / (sc.warps * 32));
     } else {
-      // grid: contiguous ranges of whole 32-word steps, at least 8 warm-ups long
+      // grid: contiguous ranges of whole 32-word steps, 8 warm-ups long where
+      // the stream has that many
       const int64_t steps = (nw + 31) / 32;
       // persistent grid: as many warps as the compiled kernel keeps resident;
       // ctas_per_sm < 0: no persistent cap, every warp takes one range of the
       // minimum length (more warps, shorter ranges, more warm-up work)
       const int64_t max_warps = sc.ctas_per_sm < 0 ? std::numeric_limits<int64_t>::max() / 2
                                                    : static_cast<int64_t>(dev.sm_count()) * per_sm * sc.warps;
-      int64_t min_range_steps = std::max<int64_t>(sc.range_steps, (pk.warm / 32) * 8);
-      int64_t warps_needed = std::max<int64_t>(1, std::min(max_warps, (steps + min_range_steps - 1) / min_range_steps));
-      range = ((steps + warps_needed - 1) / warps_needed) * 32;
+      const int64_t least = std::max<int64_t>(sc.range_steps, (pk.warm / 32) * 8);
+      range = 32 * (sc.ctas_per_sm < 0 ? least
+                                       : range_units(steps, least, max_warps,
+                                                     static_cast<int64_t>(dev.sm_count()) * kFullWarps));
       int64_t total_warps = (nw + range - 1) / range;
       blocks = static_cast<int>((total_warps + sc.warps - 1) / sc.warps);
     }

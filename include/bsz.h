@@ -68,7 +68,9 @@ typedef struct bsz_stats {
  * default schedule are {4, 64, 0, 4, 1, 0}. */
 typedef struct bsz_schedule {
   int32_t warps;        /* warps per CTA (1..16) */
-  int32_t range_steps;  /* minimum 32-word steps owned by one warp (words per tile / 32) */
+  int32_t range_steps;  /* minimum 32-word steps owned by one warp (words per tile / 32) on
+                           streams long enough to give every SM a dozen such warps; shorter
+                           streams are split into shorter ranges */
   int32_t ctas_per_sm;  /* resident CTAs per SM, 0 = as many as occupancy allows, -1 = no
                            persistent cap: one minimum-length range per warp */
   int32_t min_blocks;   /* launch-bounds minimum blocks per SM (caps registers) */
