@@ -202,19 +202,19 @@ struct Gen {
   // Global loads of one step ("load slots"): expression templates over @W@
   // (this lane's word) and @B@ (the step's first word), de-duplicated.  The
   // owned-range loop issues them one step ahead of the arithmetic.
-  std::vector<std::string> slot_tmpl;
+  std::vector<std::string> slot_tmpl, slot_fast;
   std::map<std::string, int> slot_of;
+  int64_t words_below = 0, words_above = 0;   // how far loads reach past a step's words
 
   std::string v(int n) const { return "v" + std::to_string(n); }
   bool is_input(int n) const { return in_idx.count(n) != 0; }
 
-  int slot(const std::string& tmpl) {
-    auto it = slot_of.find(tmpl);
-    if (it != slot_of.end()) return it->second;
-    int id = static_cast<int>(slot_tmpl.size());
+  // `fast`: the same load without its bounds checks
+  void slot(const std::string& tmpl, const std::string& fast) {
+    if (slot_of.count(tmpl)) return;
+    slot_of[tmpl] = static_cast<int>(slot_tmpl.size());
     slot_tmpl.push_back(tmpl);
-    slot_of[tmpl] = id;
-    return id;
+    slot_fast.push_back(fast);
   }
   static std::string subst(std::string t, const std::string& w, const std::string& b) {
     for (size_t p; (p = t.find("@W@")) != std::string::npos;) t.replace(p, 3, w);
@@ -223,34 +223,50 @@ struct Gen {
   }
   std::string slot_cur(const std::string& tmpl) const { return "cur" + std::to_string(slot_of.at(tmpl)); }
   // templates used by nodes
-  std::string t_word(int n) const { return load(n, "@W@"); }
-  std::string t_shl_lo(const Node& x) const { return load(x.a, "@W@ - " + std::to_string(x.k / 64) + "ll"); }
-  std::string t_shl_edge(const Node& x) const {
-    return "(lane == 0 ? " + load(x.a, "@B@ - " + std::to_string(x.k / 64 + 1) + "ll") + " : 0ull)";
+  std::string t_word(int n, bool fast = false) const { return load(n, "@W@", fast); }
+  std::string t_shl_lo(const Node& x, bool fast = false) const {
+    return load(x.a, x.k / 64 ? "@W@ - " + std::to_string(x.k / 64) + "ll" : "@W@", fast);
   }
-  std::string t_shr_lo(const Node& x) const { return load(x.a, "@W@ + " + std::to_string(x.k / 64) + "ll"); }
-  std::string t_shr_edge(const Node& x) const {
-    return "(lane == 31 ? " + load(x.a, "@B@ + " + std::to_string(x.k / 64 + 32) + "ll") + " : 0ull)";
+  std::string t_shl_edge(const Node& x, bool fast = false) const {
+    return "(lane == 0 ? " + load(x.a, "@B@ - " + std::to_string(x.k / 64 + 1) + "ll", fast) + " : 0ull)";
+  }
+  std::string t_shr_lo(const Node& x, bool fast = false) const {
+    return load(x.a, x.k / 64 ? "@W@ + " + std::to_string(x.k / 64) + "ll" : "@W@", fast);
+  }
+  std::string t_shr_edge(const Node& x, bool fast = false) const {
+    return "(lane == 31 ? " + load(x.a, "@B@ + " + std::to_string(x.k / 64 + 32) + "ll", fast) + " : 0ull)";
   }
   void make_slots() {
-    for (auto& kv : in_idx) slot(t_word(kv.first));
+    for (auto& kv : in_idx) slot(t_word(kv.first), t_word(kv.first, true));
     for (int n : part.order) {
       const Node& x = nodes[n];
       if (x.op == NOp::Shl && (is_input(x.a) || is_const(nodes[x.a].op))) {
-        slot(t_shl_lo(x));
-        if (x.k % 64) slot(t_shl_edge(x));
+        slot(t_shl_lo(x), t_shl_lo(x, true));
+        if (x.k % 64) slot(t_shl_edge(x), t_shl_edge(x, true));
+        words_below = std::max(words_below, x.k / 64 + 1);
       } else if (x.op == NOp::Shr) {
-        slot(t_shr_lo(x));
-        if (x.k % 64) slot(t_shr_edge(x));
+        slot(t_shr_lo(x), t_shr_lo(x, true));
+        if (x.k % 64) slot(t_shr_edge(x), t_shr_edge(x, true));
+        words_above = std::max(words_above, x.k / 64 + 1);
       }
     }
   }
+  // 32-word steps whose loads are issued together (without prefetch): a DAG
+  // of few operations is bound by memory, and one step of loads per warp at a
+  // time leaves it waiting; at most 64 registers of loaded words.
+  int block_steps() const {
+    if (part.order.size() > 48) return 1;
+    size_t n = std::max<size_t>(1, slot_tmpl.size());
+    return n <= 4 ? 8 : n <= 8 ? 4 : n <= 16 ? 2 : 1;
+  }
   // assignments of every load slot for the step starting at `b` (lane word `w`)
+  // unchecked: every word of the step's loads is known to exist
   void emit_loads(std::ostringstream& s, const std::string& prefix, bool declare, const std::string& w,
-                  const std::string& b, const char* indent) const {
+                  const std::string& b, const char* indent, bool unchecked = false,
+                  const std::string& suffix = "") const {
     for (size_t i = 0; i < slot_tmpl.size(); ++i)
-      s << indent << (declare ? "const u64 " : "") << prefix << i << " = " << subst(slot_tmpl[i], w, b)
-        << ";\n";
+      s << indent << (declare ? "const u64 " : "") << prefix << i << suffix << " = "
+        << subst(unchecked ? slot_fast[i] : slot_tmpl[i], w, b) << ";\n";
   }
 
   void analyze() {
@@ -363,7 +379,7 @@ struct Gen {
   }
 
   // expression for an input node value at word index expression `idx`
-  std::string load(int n, const std::string& idx) const {
+  std::string load(int n, const std::string& idx, bool unchecked = false) const {
     // Word `idx` of a stream; words below 0 are zero (shifting in zeros),
     // words at or past nw are the tail.
     const Node& x = nodes[n];
@@ -372,9 +388,10 @@ struct Gen {
     if (x.op == NOp::OnesMask)
       return "((" + idx + ") >= 0 && (" + idx + ") < A.nw - 1 ? ~0ull : ((" + idx +
              ") == A.nw - 1 ? A.last_mask : 0ull))";
+    const std::string word = "__ldg(A.in[" + std::to_string(in_idx.at(n)) + "] + (" + idx + "))";
+    if (unchecked) return word;
     std::string fill = x.tail ? "~0ull" : "0ull";
-    return "((" + idx + ") >= 0 && (" + idx + ") < A.nw ? __ldg(A.in[" + std::to_string(in_idx.at(n)) +
-           "] + (" + idx + ")) : " + fill + ")";
+    return "((" + idx + ") >= 0 && (" + idx + ") < A.nw ? " + word + " : " + fill + ")";
   }
 
   // value of operand o in the current step (already computed or loaded)
@@ -382,7 +399,9 @@ struct Gen {
 
   // One 32-word step.  prefetched: the load slots are already in cur<i>
   // (the owned-range loop loads them a step ahead); otherwise load here.
-  void emit_step(std::ostringstream& s, bool track, bool prefetched) const {
+  // inner: neither the stream's last word nor the range's end is in the step.
+  void emit_step(std::ostringstream& s, bool track, bool prefetched, bool inner = false) const {
+    const bool masked = this->masked && !inner;
     s << "      const long long w = base + lane;\n";
     if (masked) s << "      const u64 lm = (w == A.nw - 1) ? A.last_mask : ~0ull;\n";
     if (!prefetched) emit_loads(s, "cur", true, "w", "base", "      ");
@@ -533,7 +552,7 @@ struct Gen {
     for (int n : shl_src)
       if (!small_shl.count(n)) s << "      pv" << n << " = " << v(n) << ";\n";
     if (!track) {
-      s << "      if (w < e) {\n";
+      s << (inner ? "      {\n" : "      if (w < e) {\n");
       for (auto& kv : outs)
         s << "        " << (guard_outputs ? "if (A.out[" + std::to_string(kv.second) + "]) " : std::string())
           << "A.out[" << kv.second << "][w] = " << v(kv.first) << ";\n";
@@ -561,7 +580,8 @@ struct Gen {
     return s.str();
   }
 
-  // Whole kernel for one segment part: each warp owns range [s, e).
+  // Whole kernel for one segment part: each warp takes ranges [s, e), a whole
+  // grid's worth of them apart.
   std::string source() {
     analyze();
     std::ostringstream s;
@@ -571,10 +591,27 @@ struct Gen {
       << ")\nbsz_fused(const Args A) {\n"
       << "  const int lane = threadIdx.x & 31;\n"
       << "  const long long gw = (long long)blockIdx.x * " << warps << " + (threadIdx.x >> 5);\n"
-      << "  const long long s = gw * A.range;\n"
-      << "  if (s >= A.nw) return;\n"
+      << "  const long long stride = (long long)gridDim.x * " << warps << " * A.range;\n";
+    counters(s);
+    s << "  for (long long s = gw * A.range; s < A.nw; s += stride) {\n"
       << "  const long long e = min(s + A.range, A.nw);\n";
     body(s);
+    s << "  }\n";
+    if (!part.pops.empty()) {
+      // one atomic per CTA and popcount: with one per warp, 2^14 warps of a
+      // 2^32-bit program spent as long on their atomics as on their words
+      s << "  __shared__ unsigned long long s_pc[" << warps << "][" << part.pops.size() << "];\n"
+        << "  const int warp = threadIdx.x >> 5;\n";
+      for (size_t j = 0; j < part.pops.size(); ++j)
+        s << "  {\n    unsigned long long t = pc" << j << ";\n"
+          << "    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(~0u, t, o);\n"
+          << "    if (lane == 0) s_pc[warp][" << j << "] = t;\n  }\n";
+      s << "  __syncthreads();\n";
+      for (size_t j = 0; j < part.pops.size(); ++j)
+        s << "  if (threadIdx.x == " << j % (static_cast<size_t>(warps) * 32) << ") {\n    unsigned long long t = 0;\n    for (int k = 0; k < " << warps
+          << "; ++k) t += s_pc[k][" << j << "];\n    if (t) atomicAdd(A.slots + " << part.pops[j].second
+          << ", t);\n  }\n";
+    }
     s << "}\n";
     return s.str();
   }
@@ -588,9 +625,23 @@ struct Gen {
     s << "__device__ __noinline__ void " << name
       << "(const Args* __restrict__ Ap, const long long s, const long long e, const int lane) {\n"
       << "  const Args& A = *Ap;\n";
+    counters(s);
     body(s);
+    sums(s);
     s << "}\n";
     return s.str();
+  }
+
+  // Popcounts: per lane, then one atomic per warp.
+  void counters(std::ostringstream& s) const {
+    for (size_t j = 0; j < part.pops.size(); ++j) s << "  u32 pc" << j << " = 0;\n";
+  }
+  void sums(std::ostringstream& s) const {
+    for (size_t j = 0; j < part.pops.size(); ++j) {
+      s << "  {\n    unsigned long long t = pc" << j << ";\n"
+        << "    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(~0u, t, o);\n"
+        << "    if (lane == 0 && t) atomicAdd(A.slots + " << part.pops[j].second << ", t);\n  }\n";
+    }
   }
 
   void body(std::ostringstream& s) {
@@ -600,7 +651,6 @@ struct Gen {
     for (int i = 0; i < n_pack; ++i) s << "  u32 pk" << i << " = 0;\n";
     for (int n : shl_src)
       if (!small_shl.count(n)) s << "  u64 pv" << n << " = 0;\n";
-    for (size_t j = 0; j < part.pops.size(); ++j) s << "  u32 pc" << j << " = 0;\n";
     // ---- warm-up (speculative, exactness-checked)
     const bool need_warm = !adds.empty() || !shl_src.empty();
     if (need_warm) {
@@ -632,12 +682,33 @@ struct Gen {
         << "    p0 = s - 2 * (s - p0);\n    if (p0 < 0) p0 = 0;\n"
         << "  }\n";
     }
-    // ---- owned range: the loads of step t+1 are issued before the arithmetic
-    // of step t, so each warp keeps two steps of loads in flight.
+    // ---- owned range.  prefetch: the loads of step t+1 are issued before the
+    // arithmetic of step t, so each warp keeps two steps of loads in flight;
+    // else blocks of steps (block_steps).
     if (!prefetch) {
-      s << "  for (long long base = s; base < e; base += 32) {\n";
-      emit_step(s, false, false);
-      s << "  }\n";
+      const int U = block_steps();
+      s << "  long long base = s;\n";
+      if (U > 1) {
+        // blocks of U steps inside the stream: U steps of loads in flight
+        s << "  while (base < e) {\n    if (base >= " << words_below << " && base + " << 32 * U << " <= e && base + "
+          << 32 * U + words_above << " <= A.nw - 1) {\n      const long long base0 = base;\n";
+        for (int u = 0; u < U; ++u)
+          emit_loads(s, "ld", true, "(base0 + " + std::to_string(32 * u) + " + lane)",
+                     "(base0 + " + std::to_string(32 * u) + ")", "      ", true, "_" + std::to_string(u));
+        for (int u = 0; u < U; ++u) {
+          s << "      {\n      const long long base = base0 + " << 32 * u << ";\n";
+          for (size_t i = 0; i < slot_tmpl.size(); ++i) s << "      const u64 cur" << i << " = ld" << i << "_" << u << ";\n";
+          emit_step(s, false, true, true);
+          s << "      }\n";
+        }
+        s << "      base += " << 32 * U << ";\n    } else {\n";
+        emit_step(s, false, false);
+        s << "      base += 32;\n    }\n  }\n";
+      } else {
+        s << "  for (; base < e; base += 32) {\n";
+        emit_step(s, false, false);
+        s << "  }\n";
+      }
     } else {
     for (size_t i = 0; i < slot_tmpl.size(); ++i) s << "  u64 pf" << i << ";\n";
     s << "  {\n    const long long base = s;\n    const long long w = base + lane;\n";
@@ -651,11 +722,6 @@ struct Gen {
     s << "        }\n      }\n";
     emit_step(s, false, true);
     s << "  }\n";
-    }
-    for (size_t j = 0; j < part.pops.size(); ++j) {
-      s << "  {\n    unsigned long long t = pc" << j << ";\n"
-        << "    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(~0u, t, o);\n"
-        << "    if (lane == 0 && t) atomicAdd(A.slots + " << part.pops[j].second << ", t);\n  }\n";
     }
   }
 };
@@ -1571,6 +1637,7 @@ namespace {
 struct PartKernel {
   Compiled c;
   int64_t warm = 0;
+  bool blocked = false;   // warp form: several steps of loads at a time (a DAG bound by memory)
   // TMA form: chunk words, dynamic shared memory, resident CTAs per SM at
   // that size, and the A.in indices read through tensor maps (in map order)
   int roww = 0;
@@ -1697,6 +1764,7 @@ PartKernel part_kernel(const std::vector<Node>& nodes, const Part& p, int64_t N,
     Gen g{nodes, p, N, sc.warps, sc.min_blocks, (N % 64) != 0, sc.prefetch != 0};
     pk.c = compile_source(g.source(), sc.warps * 32, compile_ms);
     pk.warm = g.warm;
+    pk.blocked = g.block_steps() > 1;
   }
   std::lock_guard<std::mutex> lk(g_part_mu);
   part_cache()[key] = pk;
@@ -1972,20 +2040,30 @@ void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
       const int64_t total = (nw + range - 1) / range;
       blocks = static_cast<int>((total + sc.warps * 32 - 1) / (sc.warps * 32));
     } else {
-      // grid: contiguous ranges of whole 32-word steps, 8 warm-ups long where
-      // the stream has that many
+      // Contiguous ranges of whole 32-word steps, 8 warm-ups long where the
+      // stream has that many.
+      //   * ctas_per_sm 0: one range per warp, handed out in stream order, so
+      //     that the warps running at one time read and write one window of
+      //     each stream that moves along (2^32-bit long streams on a B200: 757
+      //     us in ranges of 16 steps, 848 us with one long range per resident
+      //     warp).  A DAG bound by memory takes 16 steps; one bound by its
+      //     arithmetic 64, for fewer warm-ups (a 200-op DAG of 2^29 bits: 374
+      //     us at 16, 347 us at 64); another `range_steps` is taken as given.
+      //   * > 0: that many persistent CTAs per SM, ranges a grid apart.
+      //   * < 0: ranges of the minimum length however short the stream.
       const int64_t steps = (nw + 31) / 32;
-      // persistent grid: as many warps as the compiled kernel keeps resident;
-      // ctas_per_sm < 0: no persistent cap, every warp takes one range of the
-      // minimum length (more warps, shorter ranges, more warm-up work)
-      const int64_t max_warps = sc.ctas_per_sm < 0 ? std::numeric_limits<int64_t>::max() / 2
-                                                   : static_cast<int64_t>(dev.sm_count()) * per_sm * sc.warps;
-      const int64_t least = std::max<int64_t>(sc.range_steps, (pk.warm / 32) * 8);
-      range = 32 * (sc.ctas_per_sm < 0 ? least
-                                       : range_units(steps, least, max_warps,
-                                                     static_cast<int64_t>(dev.sm_count()) * kFullWarps));
-      int64_t total_warps = (nw + range - 1) / range;
+      const int64_t resident = static_cast<int64_t>(dev.sm_count()) * per_sm * sc.warps;
+      const int64_t full = static_cast<int64_t>(dev.sm_count()) * kFullWarps;
+      int64_t least = std::max<int64_t>(sc.range_steps, (pk.warm / 32) * 8);
+      if (sc.ctas_per_sm == 0 && sc.range_steps == Schedule{}.range_steps && pk.blocked)
+        least = std::max<int64_t>(16, (pk.warm / 32) * 8);
+      int64_t r = least;
+      if (sc.ctas_per_sm == 0) r = range_units(steps, least, std::numeric_limits<int64_t>::max() / 2, std::min(resident, full));
+      else if (sc.ctas_per_sm > 0) r = range_units(steps, least, resident, full);
+      range = 32 * r;
+      const int64_t total_warps = (nw + range - 1) / range;
       blocks = static_cast<int>((total_warps + sc.warps - 1) / sc.warps);
+      if (sc.ctas_per_sm > 0) blocks = std::min<int>(blocks, dev.sm_count() * per_sm);
     }
     args[ni + no + 0] = reinterpret_cast<uint64_t>(d_slots);
     args[ni + no + 1] = reinterpret_cast<uint64_t>(impl_->d_fail + pi);

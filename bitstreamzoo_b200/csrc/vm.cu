@@ -516,7 +516,7 @@ struct Vmx {
     uint32_t g;
     asm("add.cc.u64 %0, %0, %5;\n\taddc.cc.u64 %1, %1, %6;\n\taddc.cc.u64 %2, %2, %7;\n\t"
         "addc.cc.u64 %3, %3, %8;\n\taddc.u32 %4, 0, 0;"
-        : "+l"(x[0]), "+l"(x[1]), "+l"(x[2]), "+l"(x[3]), "=r"(g)
+        : "+&l"(x[0]), "+&l"(x[1]), "+&l"(x[2]), "+&l"(x[3]), "=r"(g)
         : "l"(y[0]), "l"(y[1]), "l"(y[2]), "l"(y[3]));
     const bool p = (x[0] & x[1] & x[2] & x[3]) == ~uint64_t(0);
     const uint32_t G = __ballot_sync(0xffffffffu, g != 0), P = __ballot_sync(0xffffffffu, p);

@@ -68,11 +68,14 @@ typedef struct bsz_stats {
  * default schedule are {4, 64, 0, 4, 1, 0}. */
 typedef struct bsz_schedule {
   int32_t warps;        /* warps per CTA (1..16) */
-  int32_t range_steps;  /* minimum 32-word steps owned by one warp (words per tile / 32) on
-                           streams long enough to give every SM a dozen such warps; shorter
-                           streams are split into shorter ranges */
-  int32_t ctas_per_sm;  /* resident CTAs per SM, 0 = as many as occupancy allows, -1 = no
-                           persistent cap: one minimum-length range per warp */
+  int32_t range_steps;  /* 32-word steps owned by one warp (words per tile / 32) on streams long
+                           enough to give every SM a dozen such warps; shorter streams are split
+                           into shorter ranges.  64, the default: 16 where the DAG is bound by
+                           memory */
+  int32_t ctas_per_sm;  /* layout 0: 0 = one range per warp, in stream order; n > 0 = n persistent
+                           CTAs per SM; -1 = ranges of the full length on short streams too.
+                           Layouts 1-2: resident CTAs per SM, 0 = as many as occupancy allows, -1
+                           (layout 1) = no persistent cap */
   int32_t min_blocks;   /* launch-bounds minimum blocks per SM (caps registers) */
   int32_t prefetch;     /* 1: load the next 32-word step before computing this one */
   int32_t cut_adds;     /* carry scheme: 0, additions inside the fused kernels (speculative
