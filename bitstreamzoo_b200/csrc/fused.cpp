@@ -916,6 +916,12 @@ struct GenSeq {
            "] : " + fill + ")";
   }
 
+  // Value of an input/constant at word w of a warm-up (inside the stream).
+  std::string inside(int n) const {
+    if (is_const(nodes[n].op)) return nodes[n].op == NOp::Zero ? "0ull" : "~0ull";
+    return "__ldg(A.in[" + std::to_string(in_idx.at(n)) + "] + w)";
+  }
+
   // Value of an input/constant at the current word in the fast path.
   std::string fast_in(int n, int j) const {
     const Node& x = nodes[n];
@@ -935,15 +941,17 @@ struct GenSeq {
 
   // One word of the DAG.  mode 'f': fast (word j of the chunk at c);
   // 's': scalar at word w; 't': scalar with dirt tracking (warm-up, relative
-  // word r).  Values only; the caller stores / counts.
+  // word r; neither the stream's ends nor its last word are in a warm-up).
+  // Values only; the caller stores / counts.
   void emit_word(std::ostringstream& s, char mode, int j) const {
     const bool slow = mode != 'f';
     const std::string W = slow ? "w" : "(c + " + std::to_string(j) + ")";
+    const bool masked = this->masked && mode != 't';
     if (slow && masked) s << "      const u64 lm = (w == A.nw - 1) ? A.last_mask : ~0ull;\n";
     // every input and constant gets its value name (outputs and popcounts may
     // name a constant directly: folding can reduce an output to ZERO)
     for (auto& kv : in_idx)
-      s << "      const u64 " << v(kv.first) << " = " << (slow ? ld(kv.first, "w") : fast_in(kv.first, j)) << ";\n";
+      s << "      const u64 " << v(kv.first) << " = " << (mode == 't' ? inside(kv.first) : slow ? ld(kv.first, "w") : fast_in(kv.first, j)) << ";\n";
     auto opnd = [&](int o) -> std::string {
       if (!slow && is_const(nodes[o].op)) return fast_in(o, j);
       return v(o);
@@ -1815,6 +1823,7 @@ std::unordered_set<std::string>& spec_failed() {
 struct FusedBackend::Impl {
   Device& dev;
   ExecOptions opt;
+  bool scheduled = false;   // the caller set a schedule (else pick_form)
   BufRef fail_buf;   // from the device's buffer cache: no cudaMalloc/cudaFree per run
   unsigned int* d_fail = nullptr;   // one flag per part of the launched segment
   int64_t fail_cap = 0;
@@ -1845,10 +1854,72 @@ void FusedBackend::set_schedule(const Schedule& s) {
   c.unroll = c.unroll ? 1 : 0;
   c.shift_mul = c.shift_mul ? 1 : 0;
   impl_->opt.sched = c;
+  impl_->scheduled = true;
 }
 
+// The schedule of a segment whose caller set none: the kernel form by what
+// bounds the DAG.  The warp form moves memory best (2^29-bit MatchStar: 39 us,
+// thread forms 47-77 us) and pays about 21 instructions per addition and 12
+// per shift of a temporary for it, the thread forms 4 and 2; so it takes DAGs
+// of up to kWarpFormOps instructions per word and stream (measured on a B200
+// at 2^29 bits: long streams at 7 per stream, 109 against 170 us; the 300- and
+// 200-op DAGs at 39 and 98, 265 and 347 against 153 and 164 us), every stream
+// too short for threads (2^20 bits: equal), and what the thread forms would
+// cut into parts.  Among the thread forms 4 warps with 4-word chunks fill
+// shorter streams best (2^26 bits: 31 us, 35 us with 8-word chunks), 8-word
+// chunks carry more bytes per request on longer ones (2^29: 153 against 177
+// us), and boxes by TMA leave more issue slots to the largest DAGs (2,000-op
+// regex DAG: 186 against 210 us).
+namespace {
+
+constexpr int64_t kWarpFormOps = 20, kTmaFormOps = 25;
+constexpr int64_t kThreadFormWords = int64_t(1) << 16, kLongWords = int64_t(1) << 22;
+
+Schedule pick_form(const std::vector<Node>& nodes, const Segment& seg, int64_t nw) {
+  Schedule s;
+  s.min_blocks = 2;
+  s.prefetch = 0;
+  auto temp = [&](int o) { return o >= 0 && !nodes[o].buf && !is_const(nodes[o].op) && nodes[o].op != NOp::Buf; };
+  int64_t warp_ops = 0, thread_ops = 0;
+  bool cut = false;
+  for (int n : seg.order) {
+    const Node& x = nodes[n];
+    const bool shift = (x.op == NOp::Shl || x.op == NOp::Shr) && temp(x.a);
+    if (shift && (x.op == NOp::Shr || x.k >= 64)) cut = true;
+    warp_ops += x.op == NOp::Add ? 21 : shift ? 12 : 2;
+    thread_ops += x.op == NOp::Add ? 4 : 2;
+  }
+  int64_t streams = static_cast<int64_t>(seg.outputs.size());
+  for (int n : seg.inputs)
+    if (!is_const(nodes[n].op)) ++streams;
+  streams = std::max<int64_t>(1, streams);
+  if (cut || nw < kThreadFormWords || warp_ops <= kWarpFormOps * streams) {
+    // arithmetic-bound: the next step's loads behind this step's arithmetic
+    if (warp_ops > kWarpFormOps * streams) {
+      s.min_blocks = 4;
+      s.prefetch = 1;
+    }
+    return s;
+  }
+  s.min_blocks = 1;
+  if (nw < kLongWords) {
+    s.layout = 1;
+    s.warps = 4;
+  } else if (nw < 2 * kLongWords || thread_ops <= kTmaFormOps * streams) {
+    s.layout = 1;
+    s.warps = 8;
+    s.chunk_words = 8;
+  } else {
+    s.layout = 2;
+    s.warps = 8;
+  }
+  return s;
+}
+
+}  // namespace
+
 bool FusedBackend::all_compiled(const std::vector<Node>& nodes, const Segment& seg, int64_t N) {
-  const Schedule& sc = impl_->opt.sched;
+  const Schedule sc = impl_->scheduled ? impl_->opt.sched : pick_form(nodes, seg, (N + 63) / 64);
   {
     std::lock_guard<std::mutex> lk(g_plan_mu);
     if (plan_cache().count(graph_key(nodes, seg.order, seg.inputs, seg.outputs, seg.pops, (N % 64) != 0, sc)))
@@ -1887,8 +1958,7 @@ bool FusedBackend::all_compiled(const std::vector<Node>& nodes, const Segment& s
 void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
                        unsigned long long* d_slots, double* compile_ms) {
   Device& dev = impl_->dev;
-  const ExecOptions& opt = impl_->opt;
-  Schedule sc = opt.sched;
+  Schedule sc = impl_->scheduled ? impl_->opt.sched : pick_form(nodes, seg, nw);
   if (sc.layout >= 1) {
     // the thread-sequential forms move 32-byte sectors: every input must be
     // 32-byte aligned (the library's own buffers are 256-byte aligned; a

@@ -126,7 +126,8 @@ int64_t bsz_static_ops(bsz_program* prog, const char* const* param_names,
 bsz_run* bsz_run_create(bsz_program* prog, int64_t bitlength, int mode);
 void bsz_run_free(bsz_run* run);
 int bsz_set_param(bsz_run* run, const char* name, int64_t value);
-/* Sets the fused-kernel schedule for this run (before bsz_execute). */
+/* Sets the fused-kernel schedule for this run (before bsz_execute).  A run
+ * without one takes the kernel form that suits each segment. */
 int bsz_run_set_schedule(bsz_run* run, const bsz_schedule* schedule);
 /* Binds an input stream.  index < 0: scalar input; index >= 0: element of an
  * input array.  `words` holds n_words words on the host (on_device = 0, the
