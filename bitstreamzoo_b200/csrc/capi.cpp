@@ -14,6 +14,7 @@
 #include "fused.h"
 #include "io.h"
 #include "mlp.h"
+#include "vm.h"
 
 // Lifetimes: runs keep their program alive and programs keep their context
 // alive, so the handles may be freed in any order.
@@ -53,7 +54,7 @@ struct bsz_run {
   ~bsz_run() {
     ex.reset();
     for (cudaEvent_t e : ev)
-      if (e) cudaEventDestroy(e);
+      if (e) prog->ctx->dev->give_event(e, true);
     prog_unref(prog);
   }
 };
@@ -248,9 +249,13 @@ int bsz_bind_input(bsz_run* run, const char* name, int64_t index, const uint64_t
       else executor(run).bind_input_array(id, index, b, tail ? 1 : 0, false);
       return;
     }
-    bsz::BufRef b = dev.alloc_stream(nw);
     const int64_t have = std::min<int64_t>(static_cast<int64_t>(n_words), nw);
-    if (have > 0) {
+    // a short stream that the device interpreter will read once stays in host memory
+    const bool in_place = !on_device && nw <= bsz::kVmMaxWords &&
+                          (run->mode == BSZ_MODE_AUTO || run->mode == BSZ_MODE_VM);
+    bsz::BufRef b = in_place ? dev.host_stream(words, have, nw, tail ? ~uint64_t(0) : 0) : dev.alloc_stream(nw);
+    if (in_place) {
+    } else if (have > 0) {
       if (on_device || is_pinned(words))
         BSZ_CUDA(cudaMemcpyAsync(b->p, words, have * 8,
                                  on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
@@ -258,7 +263,7 @@ int bsz_bind_input(bsz_run* run, const char* name, int64_t index, const uint64_t
       else
         dev.h2d(b->p, words, static_cast<size_t>(have) * 8);   // pageable: staged
     }
-    if (have < nw) {
+    if (!in_place && have < nw) {
       uint64_t fill = tail ? ~uint64_t(0) : 0;
       bsz::launch_fill(dev, b->p + have, nw - have, fill, fill);
     }
@@ -290,7 +295,7 @@ static void launch_run(bsz_run* run) {
   bsz::Device& dev = *run->prog->ctx->dev;
   bsz::Executor& ex = executor(run);
   for (cudaEvent_t& e : run->ev)
-    if (!e) BSZ_CUDA(cudaEventCreate(&e));
+    if (!e) e = dev.take_event(true);
   run->l0 = dev.n_launches;
   BSZ_CUDA(cudaEventRecord(run->ev[0], dev.stream()));
   ex.run(false);
@@ -365,18 +370,18 @@ int bsz_get_stream(bsz_run* run, const char* name, int64_t index, uint64_t* host
     bsz::BufRef b = find_stream(run, name, index);
     const int64_t nw = words_of(run->bitlength);
     const int64_t n = std::min<int64_t>(nw, static_cast<int64_t>(n_words));
-    if (is_pinned(host)) {
+    if (!b->host && !b->mirror && is_pinned(host)) {
       BSZ_CUDA(cudaMemcpyAsync(host, b->p, n * 8, cudaMemcpyDeviceToHost, dev.stream()));
       dev.sync();
     } else {
-      dev.d2h(host, b->p, static_cast<size_t>(n) * 8);   // pageable: staged
+      dev.read_stream(b, n, host);   // a host copy at hand, or pageable: staged
     }
     if (n == nw && run->bitlength > 0) host[nw - 1] &= bsz::mask_for_bits(run->bitlength);
   });
 }
 
 int bsz_get_stream_device(bsz_run* run, const char* name, int64_t index, const uint64_t** dptr) {
-  return guard([&] { *dptr = find_stream(run, name, index)->p; });
+  return guard([&] { *dptr = executor(run).on_device(find_stream(run, name, index))->p; });
 }
 
 int bsz_get_int(bsz_run* run, const char* name, int64_t* value) {

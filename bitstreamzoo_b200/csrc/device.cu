@@ -22,9 +22,10 @@ Device::Device(int ordinal) : ordinal_(ordinal) {
                     std::to_string(ordinal) + " is " + prop.name);
   sm_count_ = prop.multiProcessorCount;
   BSZ_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-  BSZ_CUDA(cudaMalloc(&d_err_, 256));
-  ++n_mallocs;
-  BSZ_CUDA(cudaMemsetAsync(d_err_, 0, 256, stream_));
+  void* err = nullptr;
+  BSZ_CUDA(cudaHostAlloc(&err, 64, cudaHostAllocMapped));
+  std::memset(err, 0, 64);
+  err_ = static_cast<uint32_t*>(err);
 }
 
 Device::~Device() {
@@ -32,8 +33,11 @@ Device::~Device() {
   if (stream_) cudaStreamSynchronize(stream_);
   for (auto& kv : all_) cudaFree(kv.first);
   if (d_scan_) cudaFree(d_scan_);
-  if (d_err_) cudaFree(d_err_);
+  if (err_) cudaFreeHost(err_);
+  for (auto& pool : events_)
+    for (cudaEvent_t e : pool) cudaEventDestroy(e);
   if (d_scratch_) cudaFree(d_scratch_);
+  arena_.reset();
   for (auto& kv : *pinned_free_) cudaFreeHost(kv.second);
   pinned_free_->clear();
   for (int k = 0; k < 2; ++k) {
@@ -42,6 +46,8 @@ Device::~Device() {
   }
   if (stream_) cudaStreamDestroy(stream_);
 }
+
+constexpr size_t kMaxPinnedFree = 512;   // cached blocks; a run takes up to a few dozen
 
 std::shared_ptr<void> Device::pinned_block(size_t bytes) {
   bytes = std::max<size_t>(4096, (bytes + 4095) / 4096 * 4096);
@@ -59,7 +65,8 @@ std::shared_ptr<void> Device::pinned_block(size_t bytes) {
   // those are freed directly when the Device is gone
   std::weak_ptr<std::multimap<size_t, void*>> pool = pinned_free_;
   return std::shared_ptr<void>(p, [pool, have](void* q) {
-    if (auto m = pool.lock()) m->emplace(have, q);
+    auto m = pool.lock();
+    if (m && m->size() < kMaxPinnedFree) m->emplace(have, q);
     else cudaFreeHost(q);
   });
 }
@@ -182,6 +189,36 @@ BufRef Device::alloc_stream(int64_t n_words) {
   return s;
 }
 
+constexpr size_t kArenaBytes = size_t(256) << 10;
+
+std::shared_ptr<void> Device::host_slice(size_t bytes) {
+  bytes = (bytes + 255) & ~size_t(255);
+  if (bytes > kArenaBytes / 4) return pinned_block(bytes);
+  if (!arena_ || arena_used_ + bytes > kArenaBytes) {
+    arena_ = pinned_block(kArenaBytes);
+    arena_used_ = 0;
+  }
+  char* p = static_cast<char*>(arena_.get()) + arena_used_;
+  arena_used_ += bytes;
+  return std::shared_ptr<void>(arena_, p);
+}
+
+BufRef Device::host_stream(const uint64_t* words, int64_t have, int64_t n_words, uint64_t fill) {
+  auto s = std::make_shared<DevStream>();
+  s->host = host_slice(static_cast<size_t>(std::max<int64_t>(n_words, 1)) * 8);
+  s->p = static_cast<uint64_t*>(s->host.get());
+  s->n_words = n_words;
+  if (have > 0) std::memcpy(s->p, words, static_cast<size_t>(have) * 8);
+  for (int64_t w = have; w < n_words; ++w) s->p[w] = fill;
+  return s;
+}
+
+void Device::read_stream(const BufRef& b, int64_t n, uint64_t* out) {
+  const void* at_host = b->host ? b->p : b->mirror.get();
+  if (at_host) std::memcpy(out, at_host, static_cast<size_t>(n) * 8);
+  else d2h(out, b->p, static_cast<size_t>(n) * 8);
+}
+
 void Device::release(DevStream* s) {
   free_.emplace(s->bytes, s->p);
   bytes_live -= static_cast<int64_t>(s->bytes);
@@ -229,11 +266,32 @@ void* Device::scratch(size_t bytes) {
 }
 
 uint32_t Device::take_error() {
-  uint32_t h = 0;
-  BSZ_CUDA(cudaMemcpyAsync(&h, d_err_, 4, cudaMemcpyDeviceToHost, stream_));
   BSZ_CUDA(cudaStreamSynchronize(stream_));
-  if (h) BSZ_CUDA(cudaMemsetAsync(d_err_, 0, 4, stream_));
+  return take_error_now();
+}
+
+uint32_t Device::take_error_now() {
+  const uint32_t h = *reinterpret_cast<volatile uint32_t*>(err_);
+  if (h) *reinterpret_cast<volatile uint32_t*>(err_) = 0;
   return h;
+}
+
+cudaEvent_t Device::take_event(bool timing) {
+  auto& pool = events_[timing];
+  if (!pool.empty()) {
+    cudaEvent_t e = pool.back();
+    pool.pop_back();
+    return e;
+  }
+  cudaEvent_t e;
+  BSZ_CUDA(cudaEventCreateWithFlags(&e, timing ? cudaEventDefault : cudaEventDisableTiming));
+  return e;
+}
+
+void Device::give_event(cudaEvent_t e, bool timing) {
+  auto& pool = events_[timing];
+  if (pool.size() < 64) pool.push_back(e);
+  else cudaEventDestroy(e);
 }
 
 void Device::sync() {

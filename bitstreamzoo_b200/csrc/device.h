@@ -51,6 +51,12 @@ struct DevStream {
   int64_t n_words = 0;
   size_t bytes = 0;
   Device* dev = nullptr;
+  // Words in page-locked host memory, which kernels read in place: p points
+  // into this block (short inputs of the device interpreter).
+  std::shared_ptr<void> host;
+  // A page-locked host copy of the words, complete once the run that computed
+  // them has finished (short outputs of the device interpreter).
+  std::shared_ptr<void> mirror;
   DevStream() = default;
   DevStream(const DevStream&) = delete;
   DevStream& operator=(const DevStream&) = delete;
@@ -70,14 +76,29 @@ class Device {
   int sm_count() const { return sm_count_; }
 
   BufRef alloc_stream(int64_t n_words);
+  // A stream of n_words words in page-locked host memory that kernels read
+  // in place: words[0, have), then `fill`.  For streams read once, for which
+  // a copy to the device costs more than the read.
+  BufRef host_stream(const uint64_t* words, int64_t have, int64_t n_words, uint64_t fill);
+  // The first n words of a stream into host memory (waits for the stream's
+  // work unless a host copy is at hand: call it on finished runs).
+  void read_stream(const BufRef& b, int64_t n, uint64_t* out);
   void release(DevStream* s);
   void trim_cache();
 
   // Look-back scratch: >= n_words_needed uint32 words, zeroed on the stream.
   uint32_t* scan_state(int64_t n_u32);
-  uint32_t* error_word() const { return d_err_; }
-  // Copies the error word to the host (synchronizes the stream) and clears it.
+  // In page-locked host memory: kernels write it only on an error, so
+  // reading it costs no copy.
+  uint32_t* error_word() const { return err_; }
+  // Waits for the stream's work, reads the error word and clears it.
   uint32_t take_error();
+  // The same without the wait: errors of work known to have completed.
+  uint32_t take_error_now();
+  // Events from a pool (a run takes three; creating them costs more than
+  // recording them).
+  cudaEvent_t take_event(bool timing);
+  void give_event(cudaEvent_t e, bool timing);
   void sync();
 
   // Counters reported in the bsim_cuda JSON.
@@ -94,6 +115,9 @@ class Device {
   // from a cache (cudaHostAlloc only when none fits); it returns to the
   // cache when the last reference goes.
   std::shared_ptr<void> pinned_block(size_t bytes);
+  // A small piece of such a block (256-byte aligned); the block returns to
+  // the cache with its last piece.
+  std::shared_ptr<void> host_slice(size_t bytes);
 
   // Copies between pageable host memory and the device through two pinned
   // staging buffers: chunks are double-buffered (the host memcpy of one
@@ -120,11 +144,14 @@ class Device {
   std::vector<std::pair<void*, size_t>> all_;
   uint32_t* d_scan_ = nullptr;
   int64_t scan_cap_ = 0;
-  uint32_t* d_err_ = nullptr;
+  uint32_t* err_ = nullptr;
+  std::vector<cudaEvent_t> events_[2];
   void* d_scratch_ = nullptr;
   size_t scratch_cap_ = 0;
   void* pin_[2] = {nullptr, nullptr};
   std::shared_ptr<std::multimap<size_t, void*>> pinned_free_ = std::make_shared<std::multimap<size_t, void*>>();
+  std::shared_ptr<void> arena_;   // the block that host_slice cuts from
+  size_t arena_used_ = 0;
   cudaEvent_t pin_ev_[2] = {nullptr, nullptr};
   void ensure_pinned();
   void* raw_alloc(size_t bytes);

@@ -16,6 +16,9 @@ namespace {
 
 constexpr int kMaxWhileIters = 10000;          // simulator/pythonsim/interpreter.py:20
 constexpr int64_t kSlotChunk = 1 << 16;
+// Slots past the popcounts' capacity for the flags of one fused segment (two
+// to a slot; a segment has at most kMaxFusedOps parts).
+constexpr int64_t kFlagSlots = 1 << 12;
 // A straight-line run longer than this (unrolled loop nests reach tens of
 // millions of operations) is flushed at the next statement boundary, which
 // bounds host memory and lets the device work while the walk continues.
@@ -23,6 +26,8 @@ constexpr size_t kAutoFlushNodes = size_t(1) << 20;
 // Segments with more operations than this never become one generated
 // kernel: NVRTC time and register pressure grow with the segment.
 constexpr size_t kMaxFusedOps = 3000;
+// Host copies of outputs that the device interpreter writes (per run).
+constexpr int64_t kMaxMirrorBytes = int64_t(1) << 20;
 
 using Bits = std::vector<uint64_t>;
 inline bool bit(const Bits& b, int i) { return (b[i >> 6] >> (i & 63)) & 1u; }
@@ -218,7 +223,7 @@ Executor::~Executor() {
   // caller may free a borrowed input as soon as the run is gone).  Waiting
   // after finish() would also wait for whatever another run enqueued since.
   if (!finished_) cudaStreamSynchronize(dev_.stream());
-  if (done_ev_) cudaEventDestroy(done_ev_);
+  if (done_ev_) dev_.give_event(done_ev_, false);
   // flag, slot and VM buffers go back to the device's cache with their BufRefs
 }
 
@@ -243,6 +248,7 @@ void Executor::bind_input(int name, BufRef buf, uint8_t tail, bool clean) {
   put_raw(bind_sig_, 's');
   put_raw(bind_sig_, name);
   put_raw(bind_sig_, static_cast<uint8_t>(tail | (clean ? 2 : 0)));
+  if (buf->host) hold_.push_back(buf->host);
   var_[name] = buf_node(std::move(buf), tail, clean);
 }
 
@@ -254,6 +260,7 @@ void Executor::bind_input_array(int name, int64_t idx, BufRef buf, uint8_t tail,
   if (!arrs_[name]) arrs_[name] = std::make_unique<Arr>();
   Arr& a = *arrs_[name];
   a.defined = true;
+  if (buf->host) hold_.push_back(buf->host);
   a.elems[idx] = buf_node(std::move(buf), tail, clean);
   if (var_[name] == zero_) var_[name] = -1;   // it is an array, not a scalar input
 }
@@ -531,8 +538,20 @@ bool Executor::nonzero(int node, const Stmt* at) {
   if (n.op == NOp::OnesMask || n.op == NOp::AllOnes) return N_ > 0;
   int x = node;
   auto it = at ? live_->at.find(at->id) : live_->at.end();
+  // A value still to be computed is counted by the segment that computes it:
+  // its count, the other popcounts and the speculation flags come back in one
+  // copy, with no pass over the value of its own.
+  if (pending(node) && opt_.mode != ExecMode::Plain) {
+    ensure_slots(1);
+    const int64_t slot = n_slots_++;
+    pending_pops_.push_back({node, slot});
+    flush(it == live_->at.end() ? nullptr : &it->second, &x);
+    settle();
+    if (uint32_t err = dev_.take_error_now()) throw RuntimeError(describe_device_error(err));
+    return slot_val_[slot] != 0;
+  }
   flush(it == live_->at.end() ? nullptr : &it->second, &x);
-  if (fused_) fused_->resolve();   // the condition reads the segment's output
+  if (fused_ && fused_->pending()) settle();   // the condition reads the segment's output
   BSZ_CUDA(cudaMemsetAsync(d_flag_, 0, 4, dev_.stream()));
   launch_any(dev_, nodes_[x].buf->p, nw_, d_flag_);
   unsigned int h = 0;
@@ -624,6 +643,8 @@ void Executor::run(bool finish_now) {
       (opt_.mode == ExecMode::Vm || (opt_.mode == ExecMode::Auto && nw_ <= kVmMaxWords)) &&
       run_vm_program()) {
     ran_as_vm_program = true;
+    if (uint32_t err = dev_.take_error_now()) throw RuntimeError(describe_device_error(err));
+    finished_ = true;   // it waited for its launch
     return;
   }
   // Straight-line programs: restore a cached walk, or walk and cache it when
@@ -638,7 +659,9 @@ void Executor::run(bool finish_now) {
     exec_block(prog_.stmts);
     if (straight && n_flushes_ == f0) save_walk(key, n0);
   }
+  final_flush_ = true;
   flush(&live_->end, nullptr);
+  final_flush_ = false;
   publish_op_mix();
   // Outputs bound to constants get a buffer so the caller can read them.
   auto materialize = [&](int& node) {
@@ -661,46 +684,33 @@ void Executor::run(bool finish_now) {
 
 void Executor::enqueue_readback() {
   rb_slots_ = n_slots_ - resolved_upto_;
-  rb_flags_ = fused_ ? fused_->pending_parts() : 0;
-  readback_ = dev_.pinned_block(static_cast<size_t>(8 * rb_slots_ + 4 * rb_flags_ + 8));
-  char* h = static_cast<char*>(readback_.get());
-  if (rb_slots_ > 0)
-    BSZ_CUDA(cudaMemcpyAsync(h, d_slots_ + (resolved_upto_ - slot_base_), static_cast<size_t>(rb_slots_) * 8,
-                             cudaMemcpyDeviceToHost, dev_.stream()));
-  if (rb_flags_ > 0) fused_->enqueue_flags(reinterpret_cast<uint32_t*>(h + 8 * rb_slots_));
-  BSZ_CUDA(cudaMemcpyAsync(h + 8 * rb_slots_ + 4 * rb_flags_, dev_.error_word(), 4, cudaMemcpyDeviceToHost,
-                           dev_.stream()));
-  if (!done_ev_) BSZ_CUDA(cudaEventCreateWithFlags(&done_ev_, cudaEventDisableTiming));
+  if (published_ && published_from_ == resolved_upto_ && published_count_ == rb_slots_) {
+    readback_ = published_;
+  } else if (rb_slots_ > 0) {
+    readback_ = dev_.pinned_block(static_cast<size_t>(8 * rb_slots_));
+    BSZ_CUDA(cudaMemcpyAsync(readback_.get(), d_slots_ + (resolved_upto_ - slot_base_),
+                             static_cast<size_t>(rb_slots_) * 8, cudaMemcpyDeviceToHost, dev_.stream()));
+  }
+  if (!done_ev_) done_ev_ = dev_.take_event(false);
   BSZ_CUDA(cudaEventRecord(done_ev_, dev_.stream()));
 }
 
 void Executor::finish() {
   if (finished_) return;
-  if (readback_) {
-    // wait for this run's work and read-backs only
+  if (done_ev_) {
+    // wait for this run's work and read-back only
     BSZ_CUDA(cudaEventSynchronize(done_ev_));
-    const char* h = static_cast<const char*>(readback_.get());
-    uint32_t err = 0;
-    std::memcpy(&err, h + 8 * rb_slots_ + 4 * rb_flags_, 4);
-    const bool reran = rb_flags_ > 0 && fused_->resolve_with(reinterpret_cast<const uint32_t*>(h + 8 * rb_slots_));
-    if (!reran && rb_slots_ > 0) {
-      std::memcpy(slot_val_.data() + resolved_upto_, h, static_cast<size_t>(rb_slots_) * 8);
+    if (rb_slots_ > 0) {
+      std::memcpy(slot_val_.data() + resolved_upto_, readback_.get(), static_cast<size_t>(rb_slots_) * 8);
+      readback_.reset();
       resolved_upto_ += rb_slots_;
     }
-    readback_.reset();
-    if (err) {
-      BSZ_CUDA(cudaMemsetAsync(dev_.error_word(), 0, 4, dev_.stream()));
-      throw RuntimeError(describe_device_error(err));
-    }
-    if (!reran) {
-      finished_ = true;
-      return;
-    }
-    // a re-run rewrote popcount slots: read them again below (synchronously)
+  } else {
+    BSZ_CUDA(cudaStreamSynchronize(dev_.stream()));
   }
-  if (fused_) fused_->resolve();
-  resolve_slots();
-  if (uint32_t err = dev_.take_error()) throw RuntimeError(describe_device_error(err));
+  settle();
+  if (uint32_t err = dev_.take_error_now()) throw RuntimeError(describe_device_error(err));
+  hold_.clear();
   finished_ = true;
 }
 
@@ -715,7 +725,7 @@ void Executor::flush(const Bits* live, int* extra) {
   auto ms_since = [](clk::time_point t) { return std::chrono::duration<double, std::milli>(clk::now() - t).count(); };
   // a fused segment still pending (its speculation unchecked) must be exact
   // before anything runs after it
-  if (fused_) fused_->resolve();
+  if (fused_ && fused_->pending()) settle();
   auto t0 = clk::now();
   ++n_flushes_;
   const int n_nodes = static_cast<int>(nodes_.size());
@@ -754,15 +764,16 @@ void Executor::flush(const Bits* live, int* extra) {
     else seg.inputs.push_back(i);
   }
   for (auto& p : pending_pops_) seg.pops.push_back({p.first, p.second - slot_base_});
+  // this segment's popcount slots (allocated consecutively since the last
+  // flush) start at zero: the kernels accumulate into them
+  int64_t pop_lo = 0, n_pops = 0;
   if (!seg.pops.empty()) {
-    // this segment's popcount slots (allocated consecutively since the last
-    // flush) start at zero: the kernels accumulate into them
-    int64_t lo = seg.pops.front().second, hi = lo;
+    int64_t hi = pop_lo = seg.pops.front().second;
     for (auto& p : seg.pops) {
-      lo = std::min(lo, p.second);
+      pop_lo = std::min(pop_lo, p.second);
       hi = std::max(hi, p.second);
     }
-    BSZ_CUDA(cudaMemsetAsync(d_slots_ + lo, 0, static_cast<size_t>(hi - lo + 1) * 8, dev_.stream()));
+    n_pops = hi - pop_lo + 1;
   }
   t_segment_ms += ms_since(t0);
   if (!seg.order.empty() || !seg.pops.empty()) {
@@ -780,12 +791,31 @@ void Executor::flush(const Bits* live, int* extra) {
     }
     t_policy_ms += ms_since(t1);
     auto t2 = clk::now();
+    auto zero_slots = [&](int64_t first, int64_t n) {
+      if (n > 0) BSZ_CUDA(cudaMemsetAsync(d_slots_ + first, 0, static_cast<size_t>(n) * 8, dev_.stream()));
+    };
     if (vm) {
-      run_vm(seg);
+      run_vm(seg, pop_lo, n_pops);   // zeroes them itself
     } else if (fuse) {
+      // The parts' speculation flags take slots behind the popcounts, so
+      // that one fill clears both and one copy reads both.
+      const int64_t flag_words = (fused_->prepare(nodes_, seg, N_, nw_, &compile_ms) + 1) / 2;
+      if (slot_cap_ == 0) ensure_slots(0);
+      flags_slot_ = n_slots_;
+      const int64_t at = n_slots_ - slot_base_;
+      if (at + flag_words > slot_cap_ + kFlagSlots) throw RuntimeError("internal: no room for the parts' flags");
+      n_slots_ += flag_words;
+      if (static_cast<int64_t>(slot_val_.size()) < n_slots_) slot_val_.resize(n_slots_ + 1024);
+      if (n_pops > 0 && pop_lo + n_pops == at) {
+        zero_slots(pop_lo, n_pops + flag_words);
+      } else {
+        zero_slots(pop_lo, n_pops);
+        zero_slots(at, flag_words);
+      }
       // constants need no buffer: the generated code computes their words
-      fused_->run(nodes_, seg, N_, nw_, d_slots_, &compile_ms);
+      fused_->run(nodes_, seg, N_, nw_, d_slots_, reinterpret_cast<unsigned int*>(d_slots_ + at));
     } else {
+      zero_slots(pop_lo, n_pops);
       run_plain(seg);
     }
     t_run_ms += ms_since(t2);
@@ -882,7 +912,7 @@ bool Executor::fused_pays(const Segment& seg) {
   return fused_->all_compiled(nodes_, seg, N_);
 }
 
-void Executor::run_vm(const Segment& seg) {
+void Executor::run_vm(const Segment& seg, int64_t pop_lo, int64_t n_pops) {
   const int n_nodes = static_cast<int>(nodes_.size());
   constexpr int32_t kNone = INT32_MIN;
   std::vector<uint8_t> is_out(n_nodes, 0);
@@ -952,6 +982,23 @@ void Executor::run_vm(const Segment& seg) {
   std::stable_sort(pops.begin(), pops.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
   const int64_t kmax = 64 * nw_;
 
+  // Outputs that the caller will read are also stored to page-locked host
+  // memory while they are short, so that reading them costs no copy.
+  std::vector<uint8_t> mirrored(n_nodes, 0);
+  if (final_flush_ && nw_ <= kVmMaxWords) {
+    int64_t n = 0;
+    auto mark = [&](int x) {
+      if (x >= 0 && is_out[x] && !mirrored[x] && (n + 1) * nw_ * 8 <= kMaxMirrorBytes) {
+        mirrored[x] = 1;
+        ++n;
+      }
+    };
+    for (int id : prog_.outputs) {
+      mark(var_[id]);
+      if (arrs_[id])
+        for (auto& kv : arrs_[id]->elems) mark(kv.second);
+    }
+  }
   std::vector<VmOp> ops;
   std::vector<const uint64_t*> ext;
   int32_t n_slots = 0;
@@ -983,7 +1030,7 @@ void Executor::run_vm(const Segment& seg) {
         VmOp op{};
         op.code = kVmPop;
         op.a = loc[node];
-        op.dst = static_cast<int32_t>(it->second);
+        op.dst = static_cast<int32_t>(it->second - pop_lo);
         ops.push_back(op);
       }
     };
@@ -1023,6 +1070,7 @@ void Executor::run_vm(const Segment& seg) {
       Node& n = nodes_[id];
       const Op x = operands(id);
       if (is_out[id] && !n.buf) n.buf = dev_.alloc_stream(nw_);
+      if (is_out[id] && !in_slots) n.buf->mirror.reset();   // written only from slots
       const int32_t dst = is_out[id] && !in_slots ? ext_of(n.buf->p) : new_slot();
       loc[id] = dst;
       VmOp op{};
@@ -1054,6 +1102,13 @@ void Executor::run_vm(const Segment& seg) {
         st.dst = pointer_lo(n.buf->p);
         st.b = pointer_hi(n.buf->p);
         ops.push_back(st);
+        if (mirrored[id]) {
+          if (!n.buf->mirror) n.buf->mirror = dev_.host_slice(static_cast<size_t>(nw_) * 8);
+          const uint64_t* host = static_cast<const uint64_t*>(n.buf->mirror.get());
+          st.dst = pointer_lo(host);
+          st.b = pointer_hi(host);
+          ops.push_back(st);
+        }
       }
       emit_pops(id);
       for (int operand : {x.a, x.b}) {
@@ -1078,11 +1133,14 @@ void Executor::run_vm(const Segment& seg) {
   }
   if (ops.empty()) return;
   if (plan.ctas > 0) vm_finish(ops, n_slots, static_cast<int64_t>(ext.size()), n_loads, plan);
-  // device copies: instruction list | pointer table | slot file (if global)
+  // A short list of instructions is read in place from page-locked host
+  // memory; else device copies: instruction list | pointer table; then the
+  // value file if it is global.
   auto align = [](size_t b) { return (b + 255) & ~size_t(255); };
   const size_t ops_b = ops.size() * sizeof(VmOp);
-  const size_t ext_b = std::max<size_t>(1, ext.size()) * sizeof(uint64_t*);
-  const size_t total = align(ops_b) + align(ext_b) + static_cast<size_t>(plan.file_words) * 8;
+  const bool host_ops = plan.ctas > 0 && ext.empty() && ops.size() <= kVmWindow;
+  const size_t ops_d = host_ops ? 0 : align(ops_b), ext_d = align(ext.size() * sizeof(uint64_t*));
+  const size_t total = ops_d + ext_d + static_cast<size_t>(plan.file_words) * 8;
   if (total > vm_cap_) {
     // the old block returns to the device cache; stream order keeps it
     // alive for work already queued on it
@@ -1091,15 +1149,31 @@ void Executor::run_vm(const Segment& seg) {
     vm_buf_ = vm_mem_->p;
   }
   char* base = static_cast<char*>(vm_buf_);
-  VmOp* d_ops = reinterpret_cast<VmOp*>(base);
-  const uint64_t** d_ext = reinterpret_cast<const uint64_t**>(base + align(ops_b));
-  uint64_t* d_file =
-      plan.smem || plan.file_words == 0 ? nullptr : reinterpret_cast<uint64_t*>(base + align(ops_b) + align(ext_b));
-  BSZ_CUDA(cudaMemcpyAsync(d_ops, ops.data(), ops_b, cudaMemcpyHostToDevice, dev_.stream()));
+  const VmOp* list;
+  if (host_ops) {
+    hold_.push_back(dev_.host_slice(ops_b));
+    std::memcpy(hold_.back().get(), ops.data(), ops_b);
+    list = static_cast<const VmOp*>(hold_.back().get());
+  } else {
+    BSZ_CUDA(cudaMemcpyAsync(base, ops.data(), ops_b, cudaMemcpyHostToDevice, dev_.stream()));
+    list = reinterpret_cast<const VmOp*>(base);
+  }
+  const uint64_t** d_ext = reinterpret_cast<const uint64_t**>(base + ops_d);
   if (!ext.empty())
     BSZ_CUDA(cudaMemcpyAsync(d_ext, ext.data(), ext.size() * sizeof(uint64_t*), cudaMemcpyHostToDevice,
                              dev_.stream()));
-  VmLaunch L{d_ops, static_cast<int64_t>(ops.size()), n_loads, ext.empty() ? nullptr : d_ext, d_file, n_slots, nw_, last_mask_, d_slots_};
+  uint64_t* d_file = plan.file_words == 0 ? nullptr : reinterpret_cast<uint64_t*>(base + ops_d + ext_d);
+  VmLaunch L{list, static_cast<int64_t>(ops.size()), n_loads, ext.empty() ? nullptr : d_ext, d_file, n_slots, nw_,
+             last_mask_, d_slots_ + pop_lo};
+  L.n_pops = n_pops;
+  if (final_flush_ && plan.ctas > 0 && n_pops > 0 && n_pops <= 4096 && resolved_upto_ == slot_base_ + pop_lo &&
+      n_slots_ - resolved_upto_ == n_pops) {
+    published_ = dev_.host_slice(static_cast<size_t>(n_pops) * 8);
+    published_from_ = resolved_upto_;
+    published_count_ = n_pops;
+    L.publish = static_cast<unsigned long long*>(published_.get());
+    hold_.push_back(published_);
+  }
   launch_vm(dev_, L, plan);
   ++vm_launches;
   max_live_buffers = std::max(max_live_buffers, live_buffer_count() + n_slots);
@@ -1141,10 +1215,10 @@ void Executor::compact(int* extra) {
 void Executor::ensure_slots(int64_t need) {
   if (slot_cap_ == 0) {
     slot_cap_ = kSlotChunk;
-    slots_buf_ = dev_.alloc_stream(slot_cap_);
+    slots_buf_ = dev_.alloc_stream(slot_cap_ + kFlagSlots);
     d_slots_ = reinterpret_cast<unsigned long long*>(slots_buf_->p);
   }
-  if (n_slots_ - slot_base_ + need > slot_cap_) {
+  if (n_slots_ - slot_base_ + need > slot_cap_ - kFlagSlots) {
     resolve_slots();
     slot_base_ = n_slots_;
   }
@@ -1154,15 +1228,30 @@ void Executor::ensure_slots(int64_t need) {
 
 void Executor::resolve_slots() {
   if (!pending_pops_.empty()) flush(nullptr, nullptr);
-  if (fused_) fused_->resolve();
-  if (resolved_upto_ < n_slots_) {
-    int64_t from = resolved_upto_ - slot_base_;
-    int64_t cnt = n_slots_ - resolved_upto_;
-    BSZ_CUDA(cudaMemcpyAsync(slot_val_.data() + resolved_upto_, d_slots_ + from,
-                             static_cast<size_t>(cnt) * 8, cudaMemcpyDeviceToHost, dev_.stream()));
-    dev_.sync();
+  settle();
+}
+
+// Reads every slot not read yet (popcounts and speculation flags, one copy
+// and one wait) and re-runs what the flags say is unproven.
+void Executor::settle() {
+  auto read_from = [&](int64_t first) {
+    const size_t bytes = static_cast<size_t>(n_slots_ - first) * 8;
+    std::shared_ptr<void> block = dev_.pinned_block(bytes);
+    BSZ_CUDA(cudaMemcpyAsync(block.get(), d_slots_ + (first - slot_base_), bytes, cudaMemcpyDeviceToHost,
+                             dev_.stream()));
+    BSZ_CUDA(cudaStreamSynchronize(dev_.stream()));
+    std::memcpy(slot_val_.data() + first, block.get(), bytes);
     ++n_syncs;
+  };
+  const int64_t first = resolved_upto_;
+  if (first < n_slots_) {
+    read_from(first);
     resolved_upto_ = n_slots_;
+  }
+  if (fused_ && fused_->pending()) {
+    const bool reran = fused_->resolve_with(reinterpret_cast<const uint32_t*>(slot_val_.data() + flags_slot_));
+    // a re-run rewrote popcounts of its segment: the slots below its flags
+    if (reran) read_from(slot_base_);
   }
 }
 
@@ -1256,6 +1345,16 @@ std::shared_ptr<const Executor::Liveness> Executor::compute_liveness() const {
 }
 
 // --------------------------------------------------------------- results ---
+
+BufRef Executor::on_device(BufRef b) {
+  if (!b || !b->host) return b;
+  BufRef d = dev_.alloc_stream(nw_);
+  BSZ_CUDA(cudaMemcpyAsync(d->p, b->p, static_cast<size_t>(nw_) * 8, cudaMemcpyHostToDevice, dev_.stream()));
+  BSZ_CUDA(cudaStreamSynchronize(dev_.stream()));
+  for (Node& n : nodes_)
+    if (n.buf == b) n.buf = d;
+  return d;
+}
 
 bool Executor::has_stream(int name) const { return name >= 0 && var_[name] >= 0; }
 

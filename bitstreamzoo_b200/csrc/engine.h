@@ -115,6 +115,8 @@ class Executor {
   uint8_t stream_tail(int name) const;
   std::vector<int64_t> array_indices(int name) const;   // sorted; empty if absent
   BufRef array_value(int name, int64_t idx);
+  // The same as device memory (a short input may live in host memory).
+  BufRef on_device(BufRef b);
   bool has_array(int name) const;
   bool int_value(int name, int64_t* v);
 
@@ -187,6 +189,7 @@ class Executor {
   BufRef flag_buf_;               // cache, so a run makes no cudaMalloc/cudaFree (each
   BufRef vm_mem_;                 // cudaFree would synchronize the whole device)
   int64_t slot_cap_ = 0, slot_base_ = 0, n_slots_ = 0;
+  int64_t flags_slot_ = -1;       // first slot of the pending fused segment's flags
   std::vector<uint64_t> slot_val_;
   std::vector<std::pair<int, int64_t>> pending_pops_;
   int64_t resolved_upto_ = 0;
@@ -211,14 +214,23 @@ class Executor {
   std::string bind_sig_;
   int64_t n_flushes_ = 0;
   bool finished_ = false;         // finish() completed: no device work of this run outstanding
-  // Asynchronous run: the read-backs (popcount slots, fused speculation
-  // flags, device error word) enqueued behind the run's work into a pinned
-  // block, and an event after them; finish() waits on that event only, not
+  // Asynchronous run: the read-back (popcount slots and fused speculation
+  // flags, side by side) enqueued behind the run's work into a pinned block,
+  // and an event after it; finish() waits on that event only, not
   // on whatever other runs enqueued since.
   std::shared_ptr<void> readback_;
   cudaEvent_t done_ev_ = nullptr;
-  int64_t rb_slots_ = 0, rb_flags_ = 0;
+  int64_t rb_slots_ = 0;
   void enqueue_readback();
+  // The popcounts of the run's only segment, written to page-locked memory
+  // by the device interpreter itself (no copy).
+  std::shared_ptr<void> published_;
+  int64_t published_from_ = 0, published_count_ = 0;
+  // Page-locked blocks that enqueued kernels read or write: kept until the
+  // run has finished (the device's buffers are reused in stream order, host
+  // memory is not).
+  std::vector<std::shared_ptr<void>> hold_;
+  bool final_flush_ = false;
   ExecCache& exec_cache() const;
   std::string walk_key() const;
   bool replay_walk(const std::string& key);
@@ -255,7 +267,8 @@ class Executor {
   void flush(const std::vector<uint64_t>* live, int* extra);
   void compact(int* extra);
   void run_plain(const Segment& seg);
-  void run_vm(const Segment& seg);
+  // pop_lo, n_pops: the popcount slots that the segment accumulates into.
+  void run_vm(const Segment& seg, int64_t pop_lo, int64_t n_pops);
   // Whole program, control flow included, as one device-interpreter launch
   // (vmprog.cpp).  Returns false, with no state changed, when the program
   // needs the host during its run (see vmprog.cpp for the conditions).
@@ -265,6 +278,7 @@ class Executor {
   const uint64_t* const_ptr(int node);
   void ensure_slots(int64_t need);
   void resolve_slots();
+  void settle();
   std::shared_ptr<const Liveness> compute_liveness() const;
   int64_t live_buffer_count() const;
 };

@@ -1824,17 +1824,13 @@ struct FusedBackend::Impl {
   Device& dev;
   ExecOptions opt;
   bool scheduled = false;   // the caller set a schedule (else pick_form)
-  BufRef fail_buf;   // from the device's buffer cache: no cudaMalloc/cudaFree per run
   unsigned int* d_fail = nullptr;   // one flag per part of the launched segment
-  int64_t fail_cap = 0;
   std::unique_ptr<PendingSegment> pending;
-  Impl(Device& d, const ExecOptions& o) : dev(d), opt(o) { ensure_flags(64); }
-  void ensure_flags(int64_t n) {
-    if (n <= fail_cap) return;
-    fail_cap = std::max<int64_t>(n, 2 * fail_cap);
-    fail_buf = dev.alloc_stream((fail_cap + 1) / 2);
-    d_fail = reinterpret_cast<unsigned int*>(fail_buf->p);
-  }
+  // from prepare() to run()
+  std::shared_ptr<const SegPlan> plan;
+  Schedule plan_sched;
+  std::string plan_spec_key;
+  Impl(Device& d, const ExecOptions& o) : dev(d), opt(o) {}
 };
 
 FusedBackend::FusedBackend(Device& dev, const ExecOptions& opt)
@@ -1955,9 +1951,8 @@ bool FusedBackend::all_compiled(const std::vector<Node>& nodes, const Segment& s
 }
 
 
-void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
-                       unsigned long long* d_slots, double* compile_ms) {
-  Device& dev = impl_->dev;
+int64_t FusedBackend::prepare(const std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
+                              double* compile_ms) {
   Schedule sc = impl_->scheduled ? impl_->opt.sched : pick_form(nodes, seg, nw);
   if (sc.layout >= 1) {
     // the thread-sequential forms move 32-byte sectors: every input must be
@@ -2006,10 +2001,25 @@ void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
     plan_cache()[skey] = np;
     plan = np;
   }
-  // one speculation flag per part, read once by resolve()
   resolve();
-  impl_->ensure_flags(static_cast<int64_t>(plan->parts.size()));
-  BSZ_CUDA(cudaMemsetAsync(impl_->d_fail, 0, 4 * plan->parts.size(), dev.stream()));
+  impl_->plan = plan;
+  impl_->plan_sched = sc;
+  impl_->plan_spec_key = std::move(spec_key);
+  t_prelaunch_ms += ms_since(tp);
+  return static_cast<int64_t>(plan->parts.size());
+}
+
+void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
+                       unsigned long long* d_slots, unsigned int* d_flags) {
+  (void)seg;
+  Device& dev = impl_->dev;
+  const std::shared_ptr<const SegPlan> plan = std::move(impl_->plan);
+  const Schedule& sc = impl_->plan_sched;
+  std::string spec_key = std::move(impl_->plan_spec_key);
+  impl_->d_fail = d_flags;
+  using clk = std::chrono::steady_clock;
+  auto ms_since = [](clk::time_point t) { return std::chrono::duration<double, std::milli>(clk::now() - t).count(); };
+  auto tp = clk::now();
   for (size_t pi = 0; pi < plan->parts.size(); ++pi) {
     const Part& p = plan->parts[pi];
     const PartKernel& pk = plan->kernels[pi];
@@ -2229,16 +2239,6 @@ void FusedBackend::resolve() {
   BSZ_CUDA(cudaStreamSynchronize(dev.stream()));
   t_wait_ms += std::chrono::duration<double, std::milli>(clk::now() - tw).count();
   resolve_with(flags.data());
-}
-
-int64_t FusedBackend::pending_parts() const {
-  return impl_->pending ? static_cast<int64_t>(impl_->pending->parts->size()) : 0;
-}
-
-void FusedBackend::enqueue_flags(uint32_t* host) {
-  if (!impl_->pending) return;
-  BSZ_CUDA(cudaMemcpyAsync(host, impl_->d_fail, 4 * impl_->pending->parts->size(), cudaMemcpyDeviceToHost,
-                           impl_->dev.stream()));
 }
 
 bool FusedBackend::resolve_with(const uint32_t* flags) {

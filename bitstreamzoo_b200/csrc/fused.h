@@ -21,8 +21,11 @@ class FusedBackend {
   // the popcounts of seg.pops into d_slots[slot].  Asynchronous: the kernels
   // are enqueued with one speculation flag per part, and the segment stays
   // pending (its parts, node records and buffers held) until resolve().
+  // prepare() finds or makes the segment's plan and returns its parts, one
+  // flag each; run() launches it with `d_flags`, that many zeroed words.
+  int64_t prepare(const std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw, double* compile_ms);
   void run(std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
-           unsigned long long* d_slots, double* compile_ms);
+           unsigned long long* d_slots, unsigned int* d_flags);
   // Waits for the pending segment, reads its parts' flags and re-runs every
   // part from the first unproven one on with the exact per-op kernels (a
   // later part may have read the unproven part's outputs).  Must be called
@@ -30,12 +33,8 @@ class FusedBackend {
   // work that depends on them; a no-op when nothing is pending.
   void resolve();
   bool pending() const;
-  // Asynchronous form of resolve(): enqueue_flags copies the pending
-  // segment's flags (pending_parts() words) to pinned host memory on the
-  // stream; once that copy has completed, resolve_with(flags) re-runs what
-  // is unproven and returns true if it re-ran anything.
-  int64_t pending_parts() const;
-  void enqueue_flags(uint32_t* host);
+  // The same with the flags already read: re-runs what is unproven and
+  // returns true if it re-ran anything.
   bool resolve_with(const uint32_t* flags);
 
   void set_schedule(const Schedule& s);

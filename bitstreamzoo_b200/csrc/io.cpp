@@ -19,6 +19,7 @@
 
 #include "device.h"
 #include "engine.h"
+#include "vm.h"
 #include "frontend.h"
 
 namespace bsz {
@@ -449,7 +450,15 @@ CaseInput parse_json_case(const std::string& text) {
 // ---------------------------------------------------------------- driver ---
 namespace {
 
-BufRef upload(Device& dev, const StreamVal& v, int64_t nw) {
+// in_place: a short stream that the device interpreter will read once stays
+// in (page-locked) host memory.
+BufRef upload(Device& dev, const StreamVal& v, int64_t nw, bool in_place) {
+  if (in_place) {
+    const int64_t n = std::min<int64_t>(static_cast<int64_t>(v.n_words()), nw);
+    BufRef h = dev.host_stream(nullptr, 0, nw, v.tail ? ~uint64_t(0) : 0);
+    for (int64_t w = 0; w < n; ++w) h->p[w] = v.word(static_cast<size_t>(w));
+    return h;
+  }
   BufRef b = dev.alloc_stream(nw);
   size_t have = std::min<size_t>(v.n_words(), static_cast<size_t>(nw));
   if (have && v.view) {
@@ -490,7 +499,7 @@ bool is_clean(const StreamVal& v, int64_t N, int64_t nw) {
 
 void download(Device& dev, const BufRef& b, int64_t nw, std::vector<uint64_t>& out) {
   out.resize(nw);
-  dev.d2h(out.data(), b->p, static_cast<size_t>(nw) * 8);
+  dev.read_stream(b, nw, out.data());
 }
 
 }  // namespace
@@ -509,6 +518,7 @@ std::string run_case_json(Device& dev, const Program& prog, CaseInput& c, const 
 
   ExecOptions eo;
   eo.mode = static_cast<ExecMode>(o.mode & 3);
+  const bool in_place = nw <= kVmMaxWords && (eo.mode == ExecMode::Auto || eo.mode == ExecMode::Vm);
 
   struct OutRec {
     std::map<std::string, std::pair<std::vector<uint64_t>, uint8_t>> streams;
@@ -528,7 +538,7 @@ std::string run_case_json(Device& dev, const Program& prog, CaseInput& c, const 
       const std::string& name = prog.names[id];
       auto it = inputs.find(name);
       if (it != inputs.end()) {
-        ex->bind_input(id, upload(dev, it->second, nw), it->second.tail, is_clean(it->second, N, nw));
+        ex->bind_input(id, upload(dev, it->second, nw, in_place), it->second.tail, is_clean(it->second, N, nw));
         continue;
       }
       auto bc = c.broadcast.find(name);
@@ -536,7 +546,7 @@ std::string run_case_json(Device& dev, const Program& prog, CaseInput& c, const 
       auto ar = c.arrays.find(name);
       if (ar != c.arrays.end()) {
         for (auto& e : ar->second)
-          ex->bind_input_array(id, e.first, upload(dev, e.second, nw), e.second.tail,
+          ex->bind_input_array(id, e.first, upload(dev, e.second, nw, in_place), e.second.tail,
                                is_clean(e.second, N, nw));
       }
     }

@@ -393,6 +393,8 @@ struct VmxArgs {
   VmProgArgs prog;         // state, n_iregs: program mode only
   int64_t n_loads;
   int64_t n_slots;
+  int64_t n_pops;          // segment mode: popcounts zeroed first ...
+  unsigned long long* publish;   // ... and copied here at the end (or null)
   uint32_t unit;           // offset of slot 1 (see Vmx)
   int wpc_log2;            // words per CTA (a power of two) when there are several CTAs
 };
@@ -662,6 +664,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
                                                   m.warp * per_warp);
   uint8_t* tails = reinterpret_cast<uint8_t*>(iregs + X.prog.n_iregs);
   for (int i = m.tid; i < 2 * kMaxTotalWarps; i += m.T) (&s_ex[0][0])[i] = 0;
+  if (!PROG && m.rank == 0)
+    for (int64_t i = m.tid; i < X.n_pops; i += m.T) A.pops[i] = 0;
   if (PROG) {
     for (int64_t i = m.lane; i < X.prog.n_iregs; i += 32) iregs[i] = 0;
     for (int64_t i = m.lane; i < X.n_slots; i += 32) tails[i] = 0;
@@ -884,7 +888,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
     uint8_t* out_tails = st + 8 + 8 * X.prog.n_iregs;
     for (int64_t k = m.lane; k < X.n_slots; k += 32) out_tails[k] = tails[k];
   }
-  if (m.ctas > 1) m.barrier();   // no CTA leaves while another may read its words
+  if (m.ctas > 1 || (!PROG && X.publish)) m.barrier();   // no CTA leaves while another may read its words
+  if (!PROG && X.publish && m.rank == 0)
+    for (int64_t i = m.tid; i < X.n_pops; i += m.T) X.publish[i] = __ldcg(A.pops + i);
 }
 
 int vm_threads(int64_t nw) {
@@ -1097,8 +1103,9 @@ void launch_vm(Device& dev, const VmLaunch& L, const VmPlan& plan) {
   if (!plan.smem && !L.file && L.n_slots > 0) throw std::invalid_argument("vm: no slot file");
   ProfScope prof(dev, "k_vm");
   if (plan.ctas > 0) {
-    launch_cluster(dev, plan, false, L.ext == nullptr, VmxArgs{{a, nullptr, 0}, L.n_loads, L.n_slots, 0, 0});
+    launch_cluster(dev, plan, false, L.ext == nullptr, VmxArgs{{a, nullptr, 0}, L.n_loads, L.n_slots, L.n_pops, L.publish, 0, 0});
   } else {
+    if (L.n_pops > 0) BSZ_CUDA(cudaMemsetAsync(L.pops, 0, static_cast<size_t>(L.n_pops) * 8, dev.stream()));
     k_vm_loop<<<1, vm_threads(L.nw), 0, dev.stream()>>>(a);
     check_vm_launch(cudaGetLastError(), "vm");
   }
@@ -1112,7 +1119,7 @@ void launch_vm_program(Device& dev, const VmProgLaunch& L, const VmPlan& plan) {
   if (!plan.smem && !B.file && B.n_slots > 0) throw std::invalid_argument("vm: no slot file");
   ProfScope prof(dev, "k_vm_program");
   if (plan.ctas > 0) {
-    launch_cluster(dev, plan, true, true, VmxArgs{a, B.n_loads, B.n_slots, 0, 0});
+    launch_cluster(dev, plan, true, true, VmxArgs{a, B.n_loads, B.n_slots, 0, nullptr, 0, 0});
   } else {
     BSZ_CUDA(cudaMemsetAsync(L.state, 0, vm_state_bytes(L.n_iregs, B.n_slots), dev.stream()));
     k_vm_program_loop<<<1, vm_threads(B.nw), 0, dev.stream()>>>(a);

@@ -105,9 +105,14 @@ struct VmLaunch {
   int64_t nw;
   uint64_t last_mask;
   unsigned long long* pops;
+  // The engine zeroes pops[0, n_pops) first and, with `publish` (page-locked
+  // host memory), copies them there at the end.
+  int64_t n_pops = 0;
+  unsigned long long* publish = nullptr;
 };
 
-// Program-mode state block in device memory, read back after the launch:
+// Program-mode state block, read back after the launch (page-locked host
+// memory, written once at the end; device memory for the loop kernels):
 // [err u32, pad u32][iregs i64 x n_iregs][tails u8 x n_slots]
 struct VmProgLaunch {
   VmLaunch base;             // ops, ext, file, n_slots, nw, last_mask (pops unused)

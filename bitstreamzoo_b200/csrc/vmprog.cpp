@@ -499,16 +499,26 @@ bool Executor::run_vm_program() {
   for (auto& o : outs) {
     o.buf = dev_.alloc_stream(nw_);
     c.op(kVmStore, VmCompiler::pointer_lo(o.buf->p), o.slot, VmCompiler::pointer_hi(o.buf->p));
+    if (nw_ <= kVmMaxWords && (&o - outs.data() + 1) * nw_ * 8 <= (int64_t(1) << 20)) {
+      // a host copy, so that reading the output costs no copy
+      o.buf->mirror = dev_.host_slice(static_cast<size_t>(nw_) * 8);
+      const uint64_t* m = static_cast<const uint64_t*>(o.buf->mirror.get());
+      c.op(kVmStore, VmCompiler::pointer_lo(m), o.slot, VmCompiler::pointer_hi(m));
+    }
   }
 
-  // device buffers: instructions | state | slot file (if global)
+  // Instructions and state in page-locked host memory (the engine reads a
+  // short list in place and writes the state once, at the end); a long list,
+  // the loop kernels' state and a global value file in device memory.
   auto align = [](size_t b) { return (b + 255) & ~size_t(255); };
   const VmPlan plan = vm_plan(c.n_slots, nw_, vm_prog_warp_bytes(c.n_iregs, c.n_slots));
   vm_mark_tails(c.code, c.n_slots);
   if (plan.ctas > 0) vm_finish(c.code, c.n_slots, 0, c.n_loads, plan);
   const size_t ops_b = c.code.size() * sizeof(VmOp);
   const size_t state_b = vm_state_bytes(c.n_iregs, c.n_slots);
-  const size_t total = align(ops_b) + align(state_b) + static_cast<size_t>(plan.file_words) * 8;
+  const bool host_ops = plan.ctas > 0 && c.code.size() <= kVmWindow;
+  const size_t ops_d = host_ops ? 0 : align(ops_b), state_d = plan.ctas > 0 ? 0 : align(state_b);
+  const size_t total = ops_d + state_d + static_cast<size_t>(plan.file_words) * 8;
   if (total > vm_cap_) {
     // the old block returns to the device cache; stream order keeps it
     // alive for work already queued on it
@@ -517,20 +527,24 @@ bool Executor::run_vm_program() {
     vm_buf_ = vm_mem_->p;
   }
   char* base = static_cast<char*>(vm_buf_);
-  VmOp* d_ops = reinterpret_cast<VmOp*>(base);
-  uint8_t* d_state = reinterpret_cast<uint8_t*>(base + align(ops_b));
-  uint64_t* d_file =
-      plan.file_words == 0 ? nullptr : reinterpret_cast<uint64_t*>(base + align(ops_b) + align(state_b));
-  dev_.h2d(d_ops, c.code.data(), ops_b);
-  VmProgLaunch L{{d_ops, static_cast<int64_t>(c.code.size()), c.n_loads, nullptr, d_file, c.n_slots, nw_, last_mask_,
+  hold_.push_back(dev_.host_slice(align(state_b) + ops_b));
+  char* host = static_cast<char*>(hold_.back().get());
+  VmOp* list = reinterpret_cast<VmOp*>(host_ops ? host + align(state_b) : base);
+  if (host_ops) std::memcpy(list, c.code.data(), ops_b);
+  else dev_.h2d(list, c.code.data(), ops_b);
+  uint8_t* state = reinterpret_cast<uint8_t*>(plan.ctas > 0 ? host : base + ops_d);
+  uint64_t* d_file = plan.file_words == 0 ? nullptr : reinterpret_cast<uint64_t*>(base + ops_d + state_d);
+  VmProgLaunch L{{list, static_cast<int64_t>(c.code.size()), c.n_loads, nullptr, d_file, c.n_slots, nw_, last_mask_,
                   nullptr},
-                 d_state, c.n_iregs};
+                 state, c.n_iregs};
   launch_vm_program(dev_, L, plan);
   ++vm_launches;
   ++n_segments;
   std::vector<uint8_t> st(state_b);
-  BSZ_CUDA(cudaMemcpyAsync(st.data(), d_state, state_b, cudaMemcpyDeviceToHost, dev_.stream()));
+  if (plan.ctas == 0)
+    BSZ_CUDA(cudaMemcpyAsync(st.data(), state, state_b, cudaMemcpyDeviceToHost, dev_.stream()));
   dev_.sync();
+  if (plan.ctas > 0) std::memcpy(st.data(), host, state_b);
   ++n_syncs;
   uint32_t err = 0;
   std::memcpy(&err, st.data(), 4);
