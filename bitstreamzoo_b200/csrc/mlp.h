@@ -38,6 +38,8 @@ class Mlp {
   float* x_ = nullptr;
   float* y_ = nullptr;
   float* loss_ = nullptr;
+  float* host_ = nullptr;    // page-locked: loss, results, inputs
+  size_t host_in_ = 0;       // where the inputs start
   std::vector<float*> act_, delta_;
   int cap_ = 0;
   int64_t step_ = 0;
@@ -46,7 +48,7 @@ class Mlp {
   void ensure(int n);
   void upload(const float* x, const float* y, int n);
   void forward(int n);
-  float backward(int n);
+  void backward(int n);   // leaves the loss on its way to host_[0]
 };
 
 }  // namespace bsz
