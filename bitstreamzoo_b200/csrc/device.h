@@ -119,10 +119,9 @@ class Device {
   // the cache with its last piece.
   std::shared_ptr<void> host_slice(size_t bytes);
 
-  // Copies between pageable host memory and the device through two pinned
-  // staging buffers: chunks are double-buffered (the host memcpy of one
-  // chunk, split across threads, overlaps the DMA of the other), so large
-  // transfers run at link speed instead of the driver's pageable path.
+  // Copies between pageable host memory and the device through page-locked
+  // buffers, several threads at a time (CopyPool), so that large transfers run
+  // near link speed instead of the driver's pageable path.
   // h2d returns once `src` may be reused (the last DMA may still be in
   // flight on the stream); d2h returns with `dst` filled.  Small copies go
   // straight to cudaMemcpyAsync.
@@ -148,12 +147,11 @@ class Device {
   std::vector<cudaEvent_t> events_[2];
   void* d_scratch_ = nullptr;
   size_t scratch_cap_ = 0;
-  void* pin_[2] = {nullptr, nullptr};
   std::shared_ptr<std::multimap<size_t, void*>> pinned_free_ = std::make_shared<std::multimap<size_t, void*>>();
   std::shared_ptr<void> arena_;   // the block that host_slice cuts from
   size_t arena_used_ = 0;
-  cudaEvent_t pin_ev_[2] = {nullptr, nullptr};
-  void ensure_pinned();
+  std::unique_ptr<class CopyPool> copies_;   // made by the first large copy
+  class CopyPool& copy_pool();
   void* raw_alloc(size_t bytes);
   struct ProfRec { const char* name; cudaEvent_t a, b; };
   std::vector<ProfRec> prof_pending_;

@@ -122,3 +122,16 @@ def test_conditions_on_long_streams(ctx, nbits, unproven):
         assert np.array_equal(r.stream("acc"), want.stream("acc")), mode
         assert (r.int("n"), r.int("k")) == (want.int("n"), want.int("k")), mode
         assert r.stats["op_count"] == want.stats["op_count"]
+
+
+# words around the staged copies' 1 MiB chunk and 24-chunk ring
+@pytest.mark.parametrize("words", [1 << 17, (1 << 17) + 1, 24 << 17, (24 << 17) + 1, (50 << 17) + 3])
+def test_staged_copies(ctx, words):
+    rng = np.random.default_rng(words)
+    base = rng.integers(0, 2**64, size=words + 1, dtype=np.uint64)
+    src = "input stream a\ninput stream b\noutput stream o\noutput stream p\no = a\np = a ^ b\n"
+    a, b = base[1:], base[:-1]           # b: an address that is not 16-byte aligned with a's
+    for _ in range(3):
+        r = ctx.run(src, 64 * words, {"a": a, "b": b}, mode=bz.MODE_PLAIN)
+        assert np.array_equal(r.stream("o"), a)
+        assert np.array_equal(r.stream("p"), a ^ b)
