@@ -742,8 +742,10 @@ int bsz_op_popcount(bsz_ctx* ctx, const uint64_t* a, uint64_t n, uint64_t* resul
     auto* slot = static_cast<unsigned long long*>(dev.scratch(256));
     BSZ_CUDA(cudaMemsetAsync(slot, 0, 8, dev.stream()));
     bsz::launch_popcount(dev, a, n, slot);
-    BSZ_CUDA(cudaMemcpyAsync(result, slot, 8, cudaMemcpyDeviceToHost, dev.stream()));
+    std::shared_ptr<void> h = dev.host_slice(8);   // page-locked: one DMA, no staging
+    BSZ_CUDA(cudaMemcpyAsync(h.get(), slot, 8, cudaMemcpyDeviceToHost, dev.stream()));
     dev.sync();
+    std::memcpy(result, h.get(), 8);
   });
 }
 int bsz_s2p(bsz_ctx* ctx, const uint8_t* bytes, int64_t n_bytes, uint64_t* const* basis) {
@@ -764,10 +766,12 @@ int bsz_op_is_nonzero(bsz_ctx* ctx, const uint64_t* a, uint64_t n, int* result) 
     auto* flag = static_cast<unsigned int*>(dev.scratch(256));
     BSZ_CUDA(cudaMemsetAsync(flag, 0, 4, dev.stream()));
     bsz::launch_any(dev, a, n, flag);
-    unsigned int h = 0;
-    BSZ_CUDA(cudaMemcpyAsync(&h, flag, 4, cudaMemcpyDeviceToHost, dev.stream()));
+    std::shared_ptr<void> h = dev.host_slice(8);
+    BSZ_CUDA(cudaMemcpyAsync(h.get(), flag, 4, cudaMemcpyDeviceToHost, dev.stream()));
     dev.sync();
-    *result = h != 0;
+    unsigned int v = 0;
+    std::memcpy(&v, h.get(), 4);
+    *result = v != 0;
   });
 }
 
