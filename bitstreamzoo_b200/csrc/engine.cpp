@@ -1208,6 +1208,7 @@ void Executor::compact(int* extra) {
     if (a) for (auto& kv : a->elems) kv.second = map(kv.second);
   if (extra) *extra = map(*extra);
   nodes_after_flush_ = nodes_.size();
+  if (fused_ && fused_->pending()) fused_->keep_nodes(std::move(old));
 }
 
 // ----------------------------------------------------------------- slots ---

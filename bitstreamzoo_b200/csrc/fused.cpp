@@ -1665,15 +1665,18 @@ std::unordered_map<std::string, PartKernel>& part_cache() {
 std::string graph_key(const std::vector<Node>& nodes, const std::vector<int>& order, const std::vector<int>& inputs,
                       const std::vector<int>& outputs, const std::vector<std::pair<int, int64_t>>& pops,
                       bool masked, const Schedule& sc) {
-  std::string k;
-  k.reserve(40 * (order.size() + inputs.size()) + 16 * pops.size() + 8 * outputs.size() + 64);
-  auto put = [&](int64_t v) { k.append(reinterpret_cast<const char*>(&v), sizeof v); };
+  // written in place (this runs on every launch): 24 bytes per node
+  std::string k(24 * (order.size() + inputs.size()) + 8 * (2 * pops.size() + outputs.size() + 14), '\0');
+  char* at = &k[0];
+  auto put = [&](int64_t v) {
+    std::memcpy(at, &v, sizeof v);
+    at += sizeof v;
+  };
   auto node = [&](int n) {
     const Node& x = nodes[n];
-    put(n);
-    put(static_cast<int64_t>(x.op) | (static_cast<int64_t>(x.tail) << 8) | (static_cast<int64_t>(x.clean) << 16));
-    put(x.a);
-    put(x.b);
+    const int32_t w[4] = {n, static_cast<int32_t>(x.op) | (x.tail << 8) | (x.clean << 16), x.a, x.b};
+    std::memcpy(at, w, sizeof w);
+    at += sizeof w;
     put(x.k);
   };
   put(static_cast<int64_t>(order.size()));
@@ -1697,6 +1700,7 @@ std::string graph_key(const std::vector<Node>& nodes, const std::vector<int>& or
   put(sc.stages);
   put(sc.unroll);
   put(sc.shift_mul);
+  k.resize(static_cast<size_t>(at - k.data()));
   return k;
 }
 
@@ -1797,13 +1801,12 @@ int64_t range_units(int64_t units, int64_t least, int64_t resident, int64_t full
 constexpr int kFullWarps = 12;   // warps per SM that keep the issue slots busy (stall counters: 3.2 per scheduler)
 
 // A launched segment whose speculation flags have not been read yet: its
-// parts, a copy of every node they compute or read (with the buffers, so
-// none returns to the cache while a re-run may need it) and where its
-// popcounts go.
+// parts, the graph they are part of (with its buffers, so that none returns to
+// the cache while a re-run may need it) and where its popcounts go.
 struct PendingSegment {
   std::shared_ptr<const void> plan;          // keeps `parts` alive
   const std::vector<Part>* parts = nullptr;
-  std::unordered_map<int, Node> nodes;
+  std::vector<Node> nodes;   // the graph, once the executor gives it up (keep_nodes)
   int64_t N = 0, nw = 0;
   unsigned long long* d_slots = nullptr;
   std::string spec_key;   // non-empty: the segment ran with speculative carries (scheme 0)
@@ -2161,8 +2164,7 @@ void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
     t_prelaunch_ms += ms_since(tp);
     tp = clk::now();
   }
-  // the segment stays pending until resolve(): keep its parts and a copy of
-  // every node they compute or read, buffers included
+  // the segment stays pending until resolve()
   auto pend = std::make_unique<PendingSegment>();
   pend->plan = plan;
   pend->parts = &plan->parts;
@@ -2170,29 +2172,27 @@ void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
   pend->nw = nw;
   pend->d_slots = d_slots;
   pend->spec_key = std::move(spec_key);
-  for (const Part& p : plan->parts) {
-    for (int n : p.order) pend->nodes.emplace(n, nodes[n]);
-    for (int n : p.inputs) pend->nodes.emplace(n, nodes[n]);
-    for (auto& pp : p.pops) pend->nodes.emplace(pp.first, nodes[pp.first]);
-  }
   impl_->pending = std::move(pend);
 }
 
 bool FusedBackend::pending() const { return impl_->pending != nullptr; }
 
+void FusedBackend::keep_nodes(std::vector<Node>&& nodes) {
+  if (impl_->pending && impl_->pending->nodes.empty()) impl_->pending->nodes = std::move(nodes);
+}
+
 namespace {
 
 // Re-runs one part with the exact per-op kernels (its popcount slots are
 // cleared first), reading and writing the buffers recorded with it.
-void rerun_part_exact(Device& dev, const Part& p, std::unordered_map<int, Node>& nodes, int64_t N, int64_t nw,
+void rerun_part_exact(Device& dev, const Part& p, std::vector<Node>& nodes, int64_t N, int64_t nw,
                       unsigned long long* d_slots) {
   for (auto& pp : p.pops) BSZ_CUDA(cudaMemsetAsync(d_slots + pp.second, 0, 8, dev.stream()));
   const uint64_t lm = mask_for_bits(N);
   std::map<int, BufRef> tmp;
   auto node = [&](int n) -> Node& {
-    auto it = nodes.find(n);
-    if (it == nodes.end()) throw RuntimeError("fused re-run: a node was not recorded");
-    return it->second;
+    if (static_cast<size_t>(n) >= nodes.size()) throw RuntimeError("fused re-run: the graph was not kept");
+    return nodes[n];
   };
   auto opnd = [&](int o) -> const uint64_t* {
     const Node& y = node(o);

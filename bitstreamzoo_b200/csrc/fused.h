@@ -33,6 +33,9 @@ class FusedBackend {
   // work that depends on them; a no-op when nothing is pending.
   void resolve();
   bool pending() const;
+  // The graph of the pending segment, when its executor replaces it: kept
+  // until the segment is resolved, for a re-run.
+  void keep_nodes(std::vector<Node>&& nodes);
   // The same with the flags already read: re-runs what is unproven and
   // returns true if it re-ran anything.
   bool resolve_with(const uint32_t* flags);
