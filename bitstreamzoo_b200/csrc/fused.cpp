@@ -1269,7 +1269,9 @@ struct GenSeq {
     if (!fn_name.empty()) {
       s << "__device__ __noinline__ void " << fn_name
         << "(const Args* __restrict__ Ap, const long long s_item, const long long e_item, const int lane) {\n"
-        << "  const Args& A = *Ap;\n"
+        // its pointers in registers (220 of 255 are taken): read from memory
+        // again for every chunk they cost 8 % of a 512-instance batch
+        << "  const Args A = *Ap;\n"
         << "  const long long L = (((e_item - s_item) + 31) / 32 + " << reg_chunk - 1 << ") / " << reg_chunk << " * "
         << reg_chunk << ";\n"
         << "  const long long s = s_item + lane * L;\n"
@@ -2470,6 +2472,11 @@ BatchRunner::BatchRunner(Device& dev, const std::vector<const Program*>& progs,
   BSZ_CUDA(cudaMalloc(&m.d_ctrl, 256));
   ++dev.n_mallocs;
   std::vector<BatchItem> items;
+  const int64_t per_sm = sched.ctas_per_sm > 0 ? std::min(sched.ctas_per_sm, m.kern.blocks_per_sm)
+                                               : m.kern.blocks_per_sm;
+  const int64_t resident = dev.sm_count() * per_sm * sched.warps;
+  int64_t total_words = 0;
+  for (const BatchInstance& bi : m.inst) total_words += std::max<int64_t>(1, (bi.bitlength + 63) / 64);
   for (size_t i = 0; i < m.inst.size(); ++i) {
     const BatchInstance& bi = m.inst[i];
     if (bi.program < 0 || bi.program >= static_cast<int>(m.progs.size()))
@@ -2482,10 +2489,16 @@ BatchRunner::BatchRunner(Device& dev, const std::vector<const Program*>& progs,
     m.n_slots += static_cast<int64_t>(bp.t.pops.size());
     const int64_t nw = std::max<int64_t>(1, (bi.bitlength + 63) / 64);
     // work items: warp form, runs of 32-word steps; thread-sequential form,
-    // 32 lane ranges of whole register chunks, each at least 16 warm-ups long
+    // 32 lane ranges of whole register chunks.  16 (8) warm-ups long, shorter
+    // where all instances together would leave resident warps without an item
+    // (64 instances of up to 2^22 bits: 45 us in ranges of 64 words a lane, 35
+    // us in ranges of 24; 512 of up to 2^26: 1,017 us at 64, 1,067 at 96, 1,102
+    // at 48).
     const int64_t cw = sched.chunk_words == 8 ? 8 : 4;
-    const int64_t range = seq ? 32 * cw * ((std::max<int64_t>(64, 16 * bp.warm) + cw - 1) / cw)
-                              : 32 * std::max<int64_t>(sched.range_steps, (bp.warm / 32) * 8);
+    const int64_t no_cap = std::numeric_limits<int64_t>::max() / 2;
+    const int64_t range =
+        seq ? 32 * cw * ((range_units(total_words, std::max<int64_t>(64, 16 * bp.warm), no_cap, resident * 32) + cw - 1) / cw)
+            : 32 * range_units(total_words / 32, std::max<int64_t>(sched.range_steps, (bp.warm / 32) * 8), no_cap, resident);
     for (int64_t s0 = 0; s0 < nw; s0 += range)
       items.push_back({static_cast<int32_t>(i), bi.program, s0, std::min(nw, s0 + range)});
     uint64_t* a = args.data() + stride * i;
@@ -2511,8 +2524,6 @@ BatchRunner::BatchRunner(Device& dev, const std::vector<const Program*>& progs,
     args[stride * i + m.max_in + m.max_out] = reinterpret_cast<uint64_t>(m.d_slots + m.slot_base[i]);
   m.d_args = m.upload(args.data(), args.size() * 8);
   m.d_items = m.upload(items.data(), items.size() * sizeof(BatchItem));
-  const int64_t per_sm = sched.ctas_per_sm > 0 ? std::min(sched.ctas_per_sm, m.kern.blocks_per_sm)
-                                               : m.kern.blocks_per_sm;
   const int64_t want = (m.n_items + sched.warps - 1) / sched.warps;
   m.blocks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, dev.sm_count() * per_sm)));
   // 4. capture: reset the counters and slots, launch; replayed by launch()
