@@ -1,10 +1,11 @@
 // Fused segment backend: one generated persistent kernel per segment DAG.
 //
 // Kernel design (sm_100a, HBM-bound integer work):
-//  * The stream is split into contiguous word ranges, one per warp; a warp
-//    walks its range in 32-word steps (lane = word), so every load and store
-//    is a coalesced 256-byte warp access and only the segment's inputs and
-//    outputs touch HBM.  Every DAG temporary lives in registers.
+//  * The stream is split into contiguous word ranges, one per warp, handed out
+//    in stream order; a warp walks its range in 32-word steps (lane = word), so
+//    every load and store is a coalesced 256-byte warp access and only the
+//    segment's inputs and outputs touch HBM.  Every DAG temporary lives in
+//    registers.
 //  * Cross-word operators carry state from step to step inside the warp:
 //      - x + y: the carries of a step are resolved with two ballots and one
 //        32-bit add ((G|P) + G + carry_in); the carry out is warp-uniform;
@@ -16,14 +17,16 @@
 //    its range from an all-zero state while tracking, per node and in bits,
 //    how far the possibly-wrong ("dirty") prefix reaches (an addition is clean
 //    above the first clean bit where its operands are equal, which decides the
-//    carry; shifts move the dirt by their distance).  If the dirt has died out before the range starts the state
-//    is exact; otherwise the warm-up is doubled (up to 8 times).  If it still
-//    cannot be proven exact the kernel raises a flag and the host re-runs the
-//    segment with the plain per-op kernels, which are exact by construction.
+//    carry; shifts move the dirt by their distance).  If the dirt has died out
+//    before the range starts the state is exact; otherwise the warm-up is
+//    doubled (up to 8 times).  If it still cannot be proven exact the kernel
+//    raises a flag and the host re-runs the segment with the plain per-op
+//    kernels, which are exact by construction.
 //  * Right shifts of temporaries and left shifts of temporaries by 2048 bits
 //    or more need words the warp has not computed yet / no longer holds; the
 //    segment is cut there: the operand is materialized by an earlier kernel.
-//  * Popcounts accumulate per lane, reduce per warp, one atomic per warp.
+//  * Popcounts accumulate per lane, reduce per warp and per CTA, one atomic
+//    per CTA (batches, whose warps take items of their own: per warp).
 // Kernels are compiled with NVRTC for sm_100a and cached by their source.
 #include "fused.h"
 
@@ -620,11 +623,13 @@ struct Gen {
   std::string device_function(const std::string& name) {
     analyze();
     std::ostringstream s;
-    // the instance's argument block stays in global memory (read-only,
-    // not aliased): copying it would pin ~20 registers for the whole item
+    // The instance's argument block is copied once: read through the pointer,
+    // each chunk loads the stream addresses again before it can load a word.
+    // 512 instances of 2^18 to 2^26 bits with the default schedule: 1569 us
+    // read through the pointer, 1364 us copied.
     s << "__device__ __noinline__ void " << name
       << "(const Args* __restrict__ Ap, const long long s, const long long e, const int lane) {\n"
-      << "  const Args& A = *Ap;\n";
+      << "  const Args A = *Ap;\n";
     counters(s);
     body(s);
     sums(s);
