@@ -33,7 +33,7 @@ Device::Device(int ordinal) : ordinal_(ordinal) {
   void* err = nullptr;
   BSZ_CUDA(cudaHostAlloc(&err, 64, cudaHostAllocMapped));
   std::memset(err, 0, 64);
-  err_ = static_cast<uint32_t*>(err);
+  err_ = err_now_ = static_cast<uint32_t*>(err);
 }
 
 Device::~Device() {
@@ -377,10 +377,6 @@ void* Device::scratch(size_t bytes) {
 
 uint32_t Device::take_error() {
   BSZ_CUDA(cudaStreamSynchronize(stream_));
-  return take_error_now();
-}
-
-uint32_t Device::take_error_now() {
   const uint32_t h = *reinterpret_cast<volatile uint32_t*>(err_);
   if (h) *reinterpret_cast<volatile uint32_t*>(err_) = 0;
   return h;

@@ -88,13 +88,14 @@ class Device {
 
   // Look-back scratch: >= n_words_needed uint32 words, zeroed on the stream.
   uint32_t* scan_state(int64_t n_u32);
-  // In page-locked host memory: kernels write it only on an error, so
-  // reading it costs no copy.
-  uint32_t* error_word() const { return err_; }
-  // Waits for the stream's work, reads the error word and clears it.
+  // The word that kernels launched now report errors to, in page-locked host
+  // memory: they write it only on an error, so reading it costs no copy.  A
+  // run puts its own in place while it launches (ErrorScope), so that the
+  // error of one of several runs in flight is that run's.
+  uint32_t* error_word() const { return err_now_; }
+  // Waits for the stream's work, reads the device's own error word (per-op
+  // calls) and clears it.
   uint32_t take_error();
-  // The same without the wait: errors of work known to have completed.
-  uint32_t take_error_now();
   // Events from a pool (a run takes three; creating them costs more than
   // recording them).
   cudaEvent_t take_event(bool timing);
@@ -144,6 +145,8 @@ class Device {
   uint32_t* d_scan_ = nullptr;
   int64_t scan_cap_ = 0;
   uint32_t* err_ = nullptr;
+  uint32_t* err_now_ = nullptr;
+  friend struct ErrorScope;
   std::vector<cudaEvent_t> events_[2];
   void* d_scratch_ = nullptr;
   size_t scratch_cap_ = 0;
@@ -158,6 +161,16 @@ class Device {
   std::vector<cudaEvent_t> prof_pool_;
   std::map<std::string, std::pair<int64_t, double>> prof_totals_;
   cudaEvent_t prof_event();
+};
+
+// While it lives, kernels launched on the device report errors to `word`.
+struct ErrorScope {
+  Device& d;
+  uint32_t* before;
+  ErrorScope(Device& dev, uint32_t* word) : d(dev), before(dev.err_now_) { d.err_now_ = word; }
+  ~ErrorScope() { d.err_now_ = before; }
+  ErrorScope(const ErrorScope&) = delete;
+  ErrorScope& operator=(const ErrorScope&) = delete;
 };
 
 // Records CUDA events around one launch when the device is profiling.

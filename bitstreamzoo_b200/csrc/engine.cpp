@@ -200,6 +200,8 @@ Executor::Executor(Device& dev, const Program& prog, int64_t bitlength, ExecOpti
   if (opt_.mode != ExecMode::Plain) opt_.simplify = true;
   if (opt_.mode == ExecMode::Fused || opt_.mode == ExecMode::Auto)
     fused_ = std::make_unique<FusedBackend>(dev_, opt_);
+  err_word_ = dev_.host_slice(4);
+  *error_word() = 0;
   flag_buf_ = dev_.alloc_stream(32);
   d_flag_ = reinterpret_cast<unsigned int*>(flag_buf_->p);
   ExecCache& c = exec_cache();
@@ -547,7 +549,7 @@ bool Executor::nonzero(int node, const Stmt* at) {
     pending_pops_.push_back({node, slot});
     flush(it == live_->at.end() ? nullptr : &it->second, &x);
     settle();
-    if (uint32_t err = dev_.take_error_now()) throw RuntimeError(describe_device_error(err));
+    check_error();
     return slot_val_[slot] != 0;
   }
   flush(it == live_->at.end() ? nullptr : &it->second, &x);
@@ -558,7 +560,7 @@ bool Executor::nonzero(int node, const Stmt* at) {
   BSZ_CUDA(cudaMemcpyAsync(&h, d_flag_, 4, cudaMemcpyDeviceToHost, dev_.stream()));
   dev_.sync();
   ++n_syncs;
-  if (uint32_t err = dev_.take_error()) throw RuntimeError(describe_device_error(err));
+  check_error();
   return h != 0;
 }
 
@@ -636,6 +638,7 @@ bool has_control_flow(const std::vector<Stmt>& v) {
 }  // namespace
 
 void Executor::run(bool finish_now) {
+  ErrorScope scope(dev_, error_word());
   // Programs with if/while on short streams: the whole program, branches
   // included, runs as one launch of the device interpreter (no host round
   // trip per condition) when it qualifies.
@@ -643,7 +646,6 @@ void Executor::run(bool finish_now) {
       (opt_.mode == ExecMode::Vm || (opt_.mode == ExecMode::Auto && nw_ <= kVmMaxWords)) &&
       run_vm_program()) {
     ran_as_vm_program = true;
-    if (uint32_t err = dev_.take_error_now()) throw RuntimeError(describe_device_error(err));
     finished_ = true;   // it waited for its launch
     return;
   }
@@ -695,8 +697,14 @@ void Executor::enqueue_readback() {
   BSZ_CUDA(cudaEventRecord(done_ev_, dev_.stream()));
 }
 
+void Executor::check_error() const {
+  if (const uint32_t err = *reinterpret_cast<volatile uint32_t*>(error_word()))
+    throw RuntimeError(describe_device_error(err));
+}
+
 void Executor::finish() {
   if (finished_) return;
+  ErrorScope scope(dev_, error_word());
   if (done_ev_) {
     // wait for this run's work and read-back only
     BSZ_CUDA(cudaEventSynchronize(done_ev_));
@@ -709,7 +717,7 @@ void Executor::finish() {
     BSZ_CUDA(cudaStreamSynchronize(dev_.stream()));
   }
   settle();
-  if (uint32_t err = dev_.take_error_now()) throw RuntimeError(describe_device_error(err));
+  check_error();
   hold_.clear();
   finished_ = true;
 }
@@ -1401,6 +1409,7 @@ BufRef Executor::array_value(int name, int64_t idx) {
 
 bool Executor::int_value(int name, int64_t* v) {
   if (name < 0 || !int_def_[name]) return false;
+  ErrorScope scope(dev_, error_word());
   *v = force(ints_[name]);
   return true;
 }

@@ -230,6 +230,9 @@ class Executor {
   // run has finished (the device's buffers are reused in stream order, host
   // memory is not).
   std::vector<std::shared_ptr<void>> hold_;
+  std::shared_ptr<void> err_word_;   // this run's device error word
+  uint32_t* error_word() const { return static_cast<uint32_t*>(err_word_.get()); }
+  void check_error() const;
   bool final_flush_ = false;
   ExecCache& exec_cache() const;
   std::string walk_key() const;
