@@ -515,7 +515,7 @@ bsz_mlp* bsz_mlp_create(bsz_ctx* ctx, int in_dim, int hidden, int layers, uint64
   if (guard([&] {
         auto m = std::make_unique<bsz_mlp>();
         m->ctx = ctx;
-        m->net = std::make_unique<bsz::Mlp>(in_dim, hidden, layers, seed, ctx->dev->stream());
+        m->net = std::make_unique<bsz::Mlp>(in_dim, hidden, layers, seed, *ctx->dev);
         ++ctx->refs;
         out = m.release();
       }))

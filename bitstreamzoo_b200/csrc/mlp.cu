@@ -236,7 +236,7 @@ void set_gemm_attrs() {
 
 }  // namespace
 
-Mlp::Mlp(int in_dim, int hidden, int layers, uint64_t seed, cudaStream_t stream) : stream_(stream) {
+Mlp::Mlp(int in_dim, int hidden, int layers, uint64_t seed, Device& dev) : dev_(dev), stream_(dev.stream()) {
   if (in_dim < 1 || hidden < 1 || layers < 1) throw std::invalid_argument("mlp: bad shape");
   set_gemm_attrs();
   dims_.push_back(in_dim);
@@ -270,7 +270,6 @@ Mlp::Mlp(int in_dim, int hidden, int layers, uint64_t seed, cudaStream_t stream)
 Mlp::~Mlp() {
   cudaStreamSynchronize(stream_);
   for (float* p : {w_, g_, m_, v_, x_, y_, loss_}) if (p) cudaFree(p);
-  if (host_) cudaFreeHost(host_);
   for (float* p : act_) cudaFree(p);
   for (float* p : delta_) cudaFree(p);
 }
@@ -282,17 +281,12 @@ void Mlp::ensure(int n) {
   for (float* p : delta_) cudaFree(p);
   if (x_) cudaFree(x_);
   if (y_) cudaFree(y_);
-  if (host_) cudaFreeHost(host_);
-  x_ = y_ = host_ = nullptr;
+  x_ = y_ = nullptr;
   act_.clear();
   delta_.clear();
   cap_ = std::max(n, 256);
   check(cudaMalloc(&x_, static_cast<size_t>(cap_) * dims_[0] * 4), "mlp alloc");
   check(cudaMalloc(&y_, static_cast<size_t>(cap_) * 4), "mlp alloc");
-  // [0]: the loss; then predictions or gradients; then the inputs on their way up
-  const size_t up = static_cast<size_t>(cap_) * (dims_[0] + 1);
-  host_in_ = 1 + std::max<size_t>(static_cast<size_t>(n_params_), static_cast<size_t>(cap_));
-  check(cudaHostAlloc(&host_, 4 * (host_in_ + up), cudaHostAllocDefault), "mlp alloc");
   for (size_t l = 1; l < dims_.size(); ++l) {
     float *a = nullptr, *d = nullptr;
     check(cudaMalloc(&a, static_cast<size_t>(cap_) * dims_[l] * 4), "mlp alloc");
@@ -302,11 +296,15 @@ void Mlp::ensure(int n) {
   }
 }
 
-void Mlp::upload(const float* x, const float* y, int n) {
+// The block comes from the device's pool and goes back when the call, which
+// waits for its results, returns: one of the model's own took its first call
+// 2.5 ms to allocate.
+std::shared_ptr<float> Mlp::upload(const float* x, const float* y, int n) {
   ensure(n);
-  // earlier copies from the block are done: every call that uploads waits for
-  // its results
-  float* h = host_ + host_in_;
+  const size_t results = 1 + std::max<size_t>(static_cast<size_t>(n_params_), static_cast<size_t>(n));
+  const std::shared_ptr<void> raw = dev_.pinned_block(4 * (results + static_cast<size_t>(n) * (dims_[0] + 1)));
+  std::shared_ptr<float> block(raw, static_cast<float*>(raw.get()));
+  float* h = block.get() + results;
   const size_t nx = static_cast<size_t>(n) * dims_[0];
   std::memcpy(h, x, nx * 4);
   check(cudaMemcpyAsync(x_, h, nx * 4, cudaMemcpyHostToDevice, stream_), "mlp upload");
@@ -314,6 +312,7 @@ void Mlp::upload(const float* x, const float* y, int n) {
     std::memcpy(h + nx, y, static_cast<size_t>(n) * 4);
     check(cudaMemcpyAsync(y_, h + nx, static_cast<size_t>(n) * 4, cudaMemcpyHostToDevice, stream_), "mlp upload");
   }
+  return block;
 }
 
 void Mlp::forward(int n) {
@@ -326,7 +325,7 @@ void Mlp::forward(int n) {
   }
 }
 
-void Mlp::backward(int n) {
+void Mlp::backward(int n, float* loss) {
   const int L = static_cast<int>(dims_.size()) - 1;
   k_mse<<<1, 256, 0, stream_>>>(act_[L - 1], y_, delta_[L - 1], loss_, n);
   check(cudaGetLastError(), "mlp mse");
@@ -343,15 +342,15 @@ void Mlp::backward(int n) {
     }
   }
   ++launches;
-  check(cudaMemcpyAsync(host_, loss_, 4, cudaMemcpyDeviceToHost, stream_), "mlp loss");
+  check(cudaMemcpyAsync(loss, loss_, 4, cudaMemcpyDeviceToHost, stream_), "mlp loss");
 }
 
 float Mlp::train_step(const float* x, const float* y, int n, float lr) {
-  upload(x, y, n);
+  const std::shared_ptr<float> block = upload(x, y, n);
   forward(n);
-  backward(n);
+  backward(n, block.get());
   check(cudaStreamSynchronize(stream_), "mlp backward");
-  const float loss = host_[0];
+  const float loss = *block;
   ++step_;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, static_cast<float>(step_));
@@ -367,24 +366,24 @@ float Mlp::train_step(const float* x, const float* y, int n, float lr) {
 // Results come back through a page-locked block: a copy into the caller's
 // pageable memory by the driver takes several times as long.
 void Mlp::predict(const float* x, int n, float* out) {
-  upload(x, nullptr, n);
+  const std::shared_ptr<float> block = upload(x, nullptr, n);
   forward(n);
-  float* h = host_ + 1;
+  float* h = block.get() + 1;
   check(cudaMemcpyAsync(h, act_.back(), static_cast<size_t>(n) * 4, cudaMemcpyDeviceToHost, stream_), "mlp predict");
   check(cudaStreamSynchronize(stream_), "mlp predict");
   std::memcpy(out, h, static_cast<size_t>(n) * 4);
 }
 
 float Mlp::gradients(const float* x, const float* y, int n, float* grad) {
-  upload(x, y, n);
+  const std::shared_ptr<float> block = upload(x, y, n);
   forward(n);
-  backward(n);
-  float* h = host_ + 1;
+  backward(n, block.get());
+  float* h = block.get() + 1;
   const size_t bytes = static_cast<size_t>(n_params_) * 4;
   check(cudaMemcpyAsync(h, g_, bytes, cudaMemcpyDeviceToHost, stream_), "mlp grad");
   check(cudaStreamSynchronize(stream_), "mlp grad");
   std::memcpy(grad, h, bytes);
-  return host_[0];
+  return *block;
 }
 
 void Mlp::get_params(float* out) const {

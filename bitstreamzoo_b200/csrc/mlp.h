@@ -4,13 +4,16 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <memory>
 #include <vector>
+
+#include "device.h"
 
 namespace bsz {
 
 class Mlp {
  public:
-  Mlp(int in_dim, int hidden, int layers, uint64_t seed, cudaStream_t stream);
+  Mlp(int in_dim, int hidden, int layers, uint64_t seed, Device& dev);
   ~Mlp();
   Mlp(const Mlp&) = delete;
   Mlp& operator=(const Mlp&) = delete;
@@ -38,17 +41,18 @@ class Mlp {
   float* x_ = nullptr;
   float* y_ = nullptr;
   float* loss_ = nullptr;
-  float* host_ = nullptr;    // page-locked: loss, results, inputs
-  size_t host_in_ = 0;       // where the inputs start
   std::vector<float*> act_, delta_;
   int cap_ = 0;
   int64_t step_ = 0;
   float weight_decay_ = 0.f;
+  Device& dev_;
   cudaStream_t stream_;
   void ensure(int n);
-  void upload(const float* x, const float* y, int n);
+  // A call's page-locked block: the loss, then predictions or gradients, then
+  // the inputs, which are on their way to the device.
+  std::shared_ptr<float> upload(const float* x, const float* y, int n);
   void forward(int n);
-  void backward(int n);   // leaves the loss on its way to host_[0]
+  void backward(int n, float* loss);   // leaves the loss on its way
 };
 
 }  // namespace bsz
