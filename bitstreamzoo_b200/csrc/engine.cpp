@@ -19,6 +19,9 @@ constexpr int64_t kSlotChunk = 1 << 16;
 // Slots past the popcounts' capacity for the flags of one fused segment (two
 // to a slot; a segment has at most kMaxFusedOps parts).
 constexpr int64_t kFlagSlots = 1 << 12;
+// Slots zeroed at a time beyond those asked for, and slots that a fused kernel
+// stores to the host itself.
+constexpr int64_t kZeroAhead = 256, kMaxPublish = 128;
 // A straight-line run longer than this (unrolled loop nests reach tens of
 // millions of operations) is flushed at the next statement boundary, which
 // bounds host memory and lets the device work while the walk continues.
@@ -799,15 +802,20 @@ void Executor::flush(const Bits* live, int* extra) {
     }
     t_policy_ms += ms_since(t1);
     auto t2 = clk::now();
+    // Slots are new to every segment, so one fill serves the segments to come.
     auto zero_slots = [&](int64_t first, int64_t n) {
-      if (n > 0) BSZ_CUDA(cudaMemsetAsync(d_slots_ + first, 0, static_cast<size_t>(n) * 8, dev_.stream()));
+      if (n <= 0 || first + n <= zeroed_) return;
+      first = std::max(first, zeroed_);
+      zeroed_ = std::min(first + n + kZeroAhead, slot_cap_ + kFlagSlots);
+      BSZ_CUDA(cudaMemsetAsync(d_slots_ + first, 0, static_cast<size_t>(zeroed_ - first) * 8, dev_.stream()));
     };
     if (vm) {
       run_vm(seg, pop_lo, n_pops);   // zeroes them itself
     } else if (fuse) {
       // The parts' speculation flags take slots behind the popcounts, so
       // that one fill clears both and one copy reads both.
-      const int64_t flag_words = (fused_->prepare(nodes_, seg, N_, nw_, &compile_ms) + 1) / 2;
+      // (and the counter of the CTAs that are done, for the copy to the host).
+      const int64_t flag_words = (fused_->prepare(nodes_, seg, N_, nw_, &compile_ms) + 1) / 2 + 1;
       if (slot_cap_ == 0) ensure_slots(0);
       flags_slot_ = n_slots_;
       const int64_t at = n_slots_ - slot_base_;
@@ -821,7 +829,23 @@ void Executor::flush(const Bits* live, int* extra) {
         zero_slots(at, flag_words);
       }
       // constants need no buffer: the generated code computes their words
-      fused_->run(nodes_, seg, N_, nw_, d_slots_, reinterpret_cast<unsigned int*>(d_slots_ + at));
+      SlotPublish pub;
+      const int64_t n_pub = n_slots_ - resolved_upto_;
+      if (n_pub <= kMaxPublish) {
+        if (pub_cap_ < n_pub) {
+          pub_cap_ = std::max<int64_t>(n_pub, 32);
+          pub_buf_ = dev_.host_slice(static_cast<size_t>(pub_cap_) * 8);
+        }
+        pub.host = static_cast<unsigned long long*>(pub_buf_.get());
+        pub.from = d_slots_ + (resolved_upto_ - slot_base_);
+        pub.n = n_pub;
+        pub.done = reinterpret_cast<unsigned int*>(d_slots_ + at + flag_words - 1);
+      }
+      if (fused_->run(nodes_, seg, N_, nw_, d_slots_, reinterpret_cast<unsigned int*>(d_slots_ + at), pub)) {
+        published_ = pub_buf_;
+        published_from_ = resolved_upto_;
+        published_count_ = n_pub;
+      }
     } else {
       zero_slots(pop_lo, n_pops);
       run_plain(seg);
@@ -1230,6 +1254,7 @@ void Executor::ensure_slots(int64_t need) {
   if (n_slots_ - slot_base_ + need > slot_cap_ - kFlagSlots) {
     resolve_slots();
     slot_base_ = n_slots_;
+    zeroed_ = 0;
   }
   // (the slots a segment accumulates into are zeroed when it runs: flush())
   if (static_cast<int64_t>(slot_val_.size()) < n_slots_ + need) slot_val_.resize(n_slots_ + need + 1024);
@@ -1254,7 +1279,14 @@ void Executor::settle() {
   };
   const int64_t first = resolved_upto_;
   if (first < n_slots_) {
-    read_from(first);
+    if (published_ && published_from_ == first && published_count_ == n_slots_ - first) {
+      BSZ_CUDA(cudaStreamSynchronize(dev_.stream()));
+      std::memcpy(slot_val_.data() + first, published_.get(), static_cast<size_t>(published_count_) * 8);
+      ++n_syncs;
+    } else {
+      read_from(first);
+    }
+    published_.reset();
     resolved_upto_ = n_slots_;
   }
   if (fused_ && fused_->pending()) {

@@ -226,6 +226,9 @@ class Executor {
   // by the device interpreter itself (no copy).
   std::shared_ptr<void> published_;
   int64_t published_from_ = 0, published_count_ = 0;
+  std::shared_ptr<void> pub_buf_;    // where fused segments publish (reused)
+  int64_t pub_cap_ = 0;
+  int64_t zeroed_ = 0;               // slots below this are zero or in use
   // Page-locked blocks that enqueued kernels read or write: kept until the
   // run has finished (the device's buffers are reused in stream order, host
   // memory is not).

@@ -574,12 +574,34 @@ struct Gen {
     return std::to_string(it == sdh.end() ? 0 : it->second);
   }
 
-  static std::string args_struct(int ni, int no) {
+  // The fields at the end of a kernel's argument block: where the segment's
+  // slots go (SlotPublish), and the code that sends them.  The CTA that
+  // finishes last stores the popcounts and flags to page-locked host memory:
+  // a copy after the kernel costs the stream another 5 us before the host sees
+  // them (32 Mbit program of 12 conditions: 363 us with the copies, 291 us without).  A grid of several waves
+  // leaves `publish` null and takes the copy: each CTA's fence and ticket would
+  // hold its place from the next one.
+  static constexpr int kPublishFields = 4;
+  static std::string publish_fields() {
+    return "  u64* publish;\n  const u64* pub_from;\n  long long n_pub;\n  unsigned int* pub_done;\n";
+  }
+  static std::string publish_tail() {
+    return "  if (A.publish) {\n    __shared__ unsigned int s_last;\n"
+           "    __threadfence();   // this thread's atomics, before the CTA's ticket\n    __syncthreads();\n"
+           "    if (threadIdx.x == 0) s_last = atomicAdd(A.pub_done, 1u) == gridDim.x - 1;\n    __syncthreads();\n"
+           "    if (s_last) {\n      __threadfence();\n"
+           "      for (long long i = threadIdx.x; i < A.n_pub; i += blockDim.x) A.publish[i] = __ldcg(A.pub_from + i);\n"
+           "    }\n  }\n";
+  }
+
+  // `kernel`: of a segment's kernel, else of a batch's instances.
+  static std::string args_struct(int ni, int no, bool kernel) {
     std::ostringstream s;
     s << "typedef unsigned long long u64;\ntypedef unsigned int u32;\n"
       << "struct Args {\n  const u64* in[" << std::max(1, ni) << "];\n  u64* out[" << std::max(1, no)
       << "];\n  unsigned long long* slots;\n  unsigned int* fail;\n  long long nw;\n"
-      << "  long long range;\n  u64 last_mask;\n  unsigned long long one;\n};\n";
+      << "  long long range;\n  u64 last_mask;\n  unsigned long long one;\n"
+      << (kernel ? publish_fields() : std::string()) << "};\n";
     return s.str();
   }
 
@@ -589,7 +611,7 @@ struct Gen {
     analyze();
     std::ostringstream s;
     const int ni = static_cast<int>(part.inputs.size()), no = static_cast<int>(part.outputs.size());
-    s << args_struct(ni, no)
+    s << args_struct(ni, no, true)
       << "extern \"C\" __global__ void __launch_bounds__(" << warps * 32 << ", " << min_blocks
       << ")\nbsz_fused(const Args A) {\n"
       << "  const int lane = threadIdx.x & 31;\n"
@@ -615,7 +637,7 @@ struct Gen {
           << "; ++k) t += s_pc[k][" << j << "];\n    if (t) atomicAdd(A.slots + " << part.pops[j].second
           << ", t);\n  }\n";
     }
-    s << "}\n";
+    s << publish_tail() << "}\n";
     return s.str();
   }
 
@@ -1083,7 +1105,7 @@ struct GenSeq {
       << "struct ArgsT {\n  TMap in_map[" << std::max<size_t>(1, mapped.size()) << "];\n  TMap out_map["
       << std::max(1, no) << "];\n  const u64* in[" << std::max(1, ni) << "];\n  u64* out[" << std::max(1, no)
       << "];\n  unsigned long long* slots;\n  unsigned int* fail;\n  long long nw;\n  long long range;\n"
-      << "  u64 last_mask;\n  long long nfull;\n  unsigned long long one;\n};\n"
+      << "  u64 last_mask;\n  long long nfull;\n  unsigned long long one;\n" << Gen::publish_fields() << "};\n"
       << "__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }\n";
     return s.str();
   }
@@ -1218,7 +1240,7 @@ struct GenSeq {
     compute_mapped();
     std::ostringstream s;
     const int ni = static_cast<int>(part.inputs.size()), no = static_cast<int>(part.outputs.size());
-    s << Gen::args_struct(ni, no) << helpers();
+    s << Gen::args_struct(ni, no, true) << helpers();
     emit_kernel(s, ni, no);
     return s.str();
   }
@@ -1401,6 +1423,7 @@ struct GenSeq {
         << "    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(~0u, t, o);\n"
         << "    if (lane == 0 && t) atomicAdd(A.slots + " << part.pops[j].second << ", t);\n  }\n";
     }
+    if (fn_name.empty()) s << Gen::publish_tail();
     s << "}\n";
   }
 
@@ -2019,9 +2042,10 @@ int64_t FusedBackend::prepare(const std::vector<Node>& nodes, const Segment& seg
   return static_cast<int64_t>(plan->parts.size());
 }
 
-void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
-                       unsigned long long* d_slots, unsigned int* d_flags) {
+bool FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
+                       unsigned long long* d_slots, unsigned int* d_flags, const SlotPublish& pub) {
   (void)seg;
+  bool published = false;
   Device& dev = impl_->dev;
   const std::shared_ptr<const SegPlan> plan = std::move(impl_->plan);
   const Schedule& sc = impl_->plan_sched;
@@ -2064,7 +2088,7 @@ void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
     // argument block, laid out as the generated struct
     const int ni = std::max<int>(1, static_cast<int>(p.inputs.size()));
     const int no = std::max<int>(1, static_cast<int>(p.outputs.size()));
-    std::vector<uint64_t> args(ni + no + 6, 0);
+    std::vector<uint64_t> args(ni + no + 6 + Gen::kPublishFields, 0);
     args[ni + no + 5] = 1;   // `one`: a 1 the compiler cannot see (see GenSeq::shift_mul)
     for (size_t i = 0; i < p.inputs.size(); ++i) {
       const Node& x = nodes[p.inputs[i]];
@@ -2075,6 +2099,7 @@ void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
     int blocks = 1;
     const int per_sm = sc.ctas_per_sm > 0 ? std::min(sc.ctas_per_sm, c.blocks_per_sm) : c.blocks_per_sm;
     std::vector<uint8_t> targs;   // the TMA form's argument block
+    size_t publish_at = 0;
     if (pk.roww > 0) {
       const int R = pk.roww;
       const int per = sc.ctas_per_sm > 0 ? std::min(sc.ctas_per_sm, pk.tma_blocks_per_sm) : pk.tma_blocks_per_sm;
@@ -2088,7 +2113,7 @@ void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
       const int nm = static_cast<int>(pk.mapped.size());
       const int nmp = std::max(1, nm), nop = std::max(1, static_cast<int>(p.outputs.size()));
       const size_t maps_bytes = 128 * static_cast<size_t>(nmp + nop);
-      targs.assign(((maps_bytes + 8 * (ni + no + 7)) + 63) / 64 * 64, 0);
+      targs.assign(((maps_bytes + 8 * (ni + no + 7 + Gen::kPublishFields)) + 63) / 64 * 64, 0);
       auto encode = [&](void* dst, const uint64_t* base) {
         cuuint64_t dims[3] = {static_cast<cuuint64_t>(R), static_cast<cuuint64_t>(range / R),
                               static_cast<cuuint64_t>(nfull)};
@@ -2115,6 +2140,7 @@ void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
       tail[ni + no + 4] = mask_for_bits(N);
       tail[ni + no + 5] = static_cast<uint64_t>(nfull);
       tail[ni + no + 6] = 1;
+      publish_at = maps_bytes + 8 * static_cast<size_t>(ni + no + 7);
     } else if (sc.layout >= 1) {
       // thread-sequential: one range of whole register chunks per thread, 16
       // warm-ups long where the stream has that many; a persistent grid of
@@ -2160,6 +2186,15 @@ void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
     args[ni + no + 2] = static_cast<uint64_t>(nw);
     args[ni + no + 3] = static_cast<uint64_t>(range);
     args[ni + no + 4] = mask_for_bits(N);
+    const int resident = pk.roww > 0 ? pk.tma_blocks_per_sm : c.blocks_per_sm;
+    if (pi + 1 == plan->parts.size() && pub.n > 0 && blocks <= static_cast<int64_t>(dev.sm_count()) * resident) {
+      uint64_t* f = pk.roww > 0 ? reinterpret_cast<uint64_t*>(targs.data() + publish_at) : args.data() + ni + no + 6;
+      f[0] = reinterpret_cast<uint64_t>(pub.host);
+      f[1] = reinterpret_cast<uint64_t>(pub.from);
+      f[2] = static_cast<uint64_t>(pub.n);
+      f[3] = reinterpret_cast<uint64_t>(pub.done);
+      published = true;
+    }
     void* kparams[] = {pk.roww > 0 ? static_cast<void*>(targs.data()) : static_cast<void*>(args.data())};
     {
       ProfScope prof(dev, "fused");
@@ -2180,6 +2215,7 @@ void FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
   pend->d_slots = d_slots;
   pend->spec_key = std::move(spec_key);
   impl_->pending = std::move(pend);
+  return published;
 }
 
 bool FusedBackend::pending() const { return impl_->pending != nullptr; }
@@ -2454,7 +2490,7 @@ BatchRunner::BatchRunner(Device& dev, const std::vector<const Program*>& progs,
   }
   // 2. one kernel: every program's DAG as a device function + a work loop
   std::ostringstream src;
-  src << Gen::args_struct(m.max_in, m.max_out) << (seq ? GenSeq::helpers() : std::string()) << fns
+  src << Gen::args_struct(m.max_in, m.max_out, false) << (seq ? GenSeq::helpers() : std::string()) << fns
       << "struct Item { int inst; int dag; long long s; long long e; };\n"
       << "extern \"C\" __global__ void __launch_bounds__(" << sched.warps * 32 << ", "
       << sched.min_blocks << ")\nbsz_batch(const Args* __restrict__ insts, "

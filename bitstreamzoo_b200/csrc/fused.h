@@ -13,6 +13,15 @@
 
 namespace bsz {
 
+// Where a segment's slots go when its last kernel hands them to the host
+// itself: n words from `from` to `host` (page-locked), `done` a zeroed counter.
+struct SlotPublish {
+  unsigned long long* host = nullptr;
+  const unsigned long long* from = nullptr;
+  int64_t n = 0;
+  unsigned int* done = nullptr;
+};
+
 class FusedBackend {
  public:
   FusedBackend(Device& dev, const ExecOptions& opt);
@@ -22,10 +31,12 @@ class FusedBackend {
   // are enqueued with one speculation flag per part, and the segment stays
   // pending (its parts, node records and buffers held) until resolve().
   // prepare() finds or makes the segment's plan and returns its parts, one
-  // flag each; run() launches it with `d_flags`, that many zeroed words.
+  // flag each; run() launches it with `d_flags`, that many zeroed words, and
+  // returns true if its last kernel does what `pub` says (not when that is a
+  // carry scan, or a grid of more than one wave).
   int64_t prepare(const std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw, double* compile_ms);
-  void run(std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
-           unsigned long long* d_slots, unsigned int* d_flags);
+  bool run(std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
+           unsigned long long* d_slots, unsigned int* d_flags, const SlotPublish& pub);
   // Waits for the pending segment, reads its parts' flags and re-runs every
   // part from the first unproven one on with the exact per-op kernels (a
   // later part may have read the unproven part's outputs).  Must be called
