@@ -17,6 +17,7 @@
 //   POPCOUNT                one pass, one atomic per CTA, no host sync
 //   ANY                     stops reading once a set bit has been seen
 #include "device.h"
+#include "pdl.cuh"
 
 #include <algorithm>
 
@@ -67,6 +68,7 @@ template <int OP>
 __global__ void __launch_bounds__(kThreads)
 k_map_vec(uint64_t* __restrict__ d, const uint64_t* __restrict__ a, const uint64_t* __restrict__ b,
           int64_t n, uint64_t last_mask) {
+  after_previous(a, b);
   const int64_t nvec = (n - 1) / 2;
   const ulonglong2* A = reinterpret_cast<const ulonglong2*>(a);
   const ulonglong2* B = reinterpret_cast<const ulonglong2*>(b);
@@ -107,6 +109,7 @@ k_map_vec(uint64_t* __restrict__ d, const uint64_t* __restrict__ a, const uint64
 template <int OP>
 __global__ void __launch_bounds__(kThreads)
 k_map_scalar(uint64_t* d, const uint64_t* a, const uint64_t* b, int64_t n, uint64_t last_mask) {
+  after_previous(a, b);
   const int64_t step = static_cast<int64_t>(gridDim.x) * kThreads;
   for (int64_t w = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x; w < n; w += step) {
     uint64_t r = apply_any<OP>(a[w], OP != 4 ? b[w] : 0);
@@ -125,10 +128,10 @@ void launch_map(Device& dev, uint64_t* d, const uint64_t* a, const uint64_t* b, 
   if (vec) {
     int64_t nvec = (n - 1) / 2;
     const unsigned grid = grid_in_order(std::max<int64_t>(nvec, 1), kThreads * kUnroll);
-    k_map_vec<OP><<<grid, kThreads, 0, dev.stream()>>>(d, a, b, n, last_mask);
+    launch_after(dev.stream(), grid, kThreads, 0, k_map_vec<OP>, d, a, b, n, last_mask);
   } else {
     int grid = grid_for(dev, n, kThreads);
-    k_map_scalar<OP><<<grid, kThreads, 0, dev.stream()>>>(d, a, b, n, last_mask);
+    launch_after(dev.stream(), grid, kThreads, 0, k_map_scalar<OP>, d, a, b, n, last_mask);
   }
   check_launch();
   ++dev.n_launches;
@@ -150,6 +153,7 @@ template <bool LEFT>
 __global__ void __launch_bounds__(kThreads)
 k_shift(uint64_t* __restrict__ d, const uint64_t* __restrict__ a, int64_t ws, int bs, int64_t n,
         uint64_t last_mask, uint64_t fill) {
+  after_previous(a);
   const int lane = threadIdx.x & 31;
   const int64_t warps = static_cast<int64_t>(gridDim.x) * (kThreads / 32);
   auto source = [&](int64_t w) -> uint64_t {
@@ -285,6 +289,7 @@ __global__ void __launch_bounds__(kAddWarps * 32, kAddMinBlocks)
 k_add(uint64_t* d, const uint64_t* a, const uint64_t* b, int64_t n, uint64_t last_mask,
       uint32_t* __restrict__ state, uint32_t* __restrict__ err, int in_place, int64_t silent_tile,
       int spin_limit) {
+  after_previous(a, b, state);
   __shared__ uint32_t s_ticket;
   if (threadIdx.x == 0) s_ticket = atomicAdd(&state[0], 1u);
   __syncthreads();
@@ -366,6 +371,7 @@ __device__ __forceinline__ uint64_t warp_sum(uint64_t v) {
 __global__ void __launch_bounds__(kThreads)
 k_popcount(const uint64_t* __restrict__ a, int64_t n, unsigned long long* __restrict__ slot,
            int vec) {
+  after_previous(a);
   __shared__ uint64_t s_part[kThreads / 32];
   uint64_t c = 0;
   if (vec) {
@@ -408,6 +414,7 @@ constexpr int kAnyUnroll = 8;
 
 __global__ void __launch_bounds__(kThreads)
 k_any(const uint64_t* __restrict__ a, int64_t n, unsigned int* flag, int vec) {
+  after_previous(a);
   const int64_t items = vec ? n / 2 : n;
   const ulonglong2* A = reinterpret_cast<const ulonglong2*>(a);
   const int64_t step = static_cast<int64_t>(gridDim.x) * kThreads * kAnyUnroll;
@@ -439,6 +446,7 @@ k_any(const uint64_t* __restrict__ a, int64_t n, unsigned int* flag, int vec) {
 
 __global__ void __launch_bounds__(kThreads)
 k_fill(uint64_t* __restrict__ d, int64_t n, uint64_t value, uint64_t last_value) {
+  after_previous(d);
   const int64_t step = static_cast<int64_t>(gridDim.x) * kThreads;
   for (int64_t w = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x; w < n; w += step)
     d[w] = (w == n - 1) ? last_value : value;
@@ -467,8 +475,8 @@ void launch_shl(Device& dev, uint64_t* d, const uint64_t* a, int64_t k, int64_t 
   int64_t ws = std::min<int64_t>(k / 64, n + 1);
   int bs = static_cast<int>(k % 64);
   ProfScope prof(dev, "k_shl");
-  k_shift<true><<<grid_in_order(n, kShiftTile * (kThreads / 32)), kThreads, 0, dev.stream()>>>(d, a, ws, bs, n,
-                                                                                              last_mask, 0);
+  launch_after(dev.stream(), grid_in_order(n, kShiftTile * (kThreads / 32)), kThreads, 0, k_shift<true>, d, a, ws, bs,
+               n, last_mask, 0);
   check_launch();
   ++dev.n_launches;
 }
@@ -478,8 +486,8 @@ void launch_shr(Device& dev, uint64_t* d, const uint64_t* a, int64_t k, int64_t 
   int64_t ws = std::min<int64_t>(k / 64, n + 1);
   int bs = static_cast<int>(k % 64);
   ProfScope prof(dev, "k_shr");
-  k_shift<false><<<grid_in_order(n, kShiftTile * (kThreads / 32)), kThreads, 0, dev.stream()>>>(d, a, ws, bs, n,
-                                                                                               ~uint64_t(0), fill);
+  launch_after(dev.stream(), grid_in_order(n, kShiftTile * (kThreads / 32)), kThreads, 0, k_shift<false>, d, a, ws, bs,
+               n, ~uint64_t(0), fill);
   check_launch();
   ++dev.n_launches;
 }
@@ -487,15 +495,19 @@ void launch_shr(Device& dev, uint64_t* d, const uint64_t* a, int64_t k, int64_t 
 int64_t add_state_words(int64_t n) { return 1 + (n + kAddTile - 1) / kAddTile; }
 
 static void launch_add_kernel(cudaStream_t stream, uint64_t* d, const uint64_t* a, const uint64_t* b,
-                              int64_t n, uint64_t last_mask, uint32_t* state, uint32_t* err) {
+                              int64_t n, uint64_t last_mask, uint32_t* state, uint32_t* err, bool own_stream) {
   const int64_t tiles = (n + kAddTile - 1) / kAddTile;
   if (tiles > 0x7fffffff) throw std::invalid_argument("launch_add: stream too long");
   const int in_place = (d == a || d == b) ? 1 : 0;
   // one warp per tile, one ticket per CTA of kAddWarps tiles
   const int64_t blocks = (tiles + kAddWarps - 1) / kAddWarps;
   if (blocks > 0x7fffffff) throw std::invalid_argument("launch_add: stream too long");
-  k_add<<<static_cast<unsigned>(blocks), kAddWarps * 32, 0, stream>>>(d, a, b, n, last_mask, state, err, in_place,
-                                                                      g_add_silent_tile, g_add_spin_limit);
+  if (own_stream)
+    launch_after(stream, static_cast<unsigned>(blocks), kAddWarps * 32, 0, k_add, d, a, b, n, last_mask, state, err,
+                 in_place, g_add_silent_tile, g_add_spin_limit);
+  else
+    k_add<<<static_cast<unsigned>(blocks), kAddWarps * 32, 0, stream>>>(d, a, b, n, last_mask, state, err, in_place,
+                                                                        g_add_silent_tile, g_add_spin_limit);
   check_launch();
 }
 
@@ -503,14 +515,14 @@ void launch_add_with_state(Device& dev, uint64_t* d, const uint64_t* a, const ui
                            int64_t n, uint64_t last_mask, uint32_t* state) {
   if (n <= 0) return;
   ProfScope prof(dev, "k_add");
-  launch_add_kernel(dev.stream(), d, a, b, n, last_mask, state, dev.error_word());
+  launch_add_kernel(dev.stream(), d, a, b, n, last_mask, state, dev.error_word(), true);
   ++dev.n_launches;
 }
 
 void launch_add_on_stream(cudaStream_t stream, uint64_t* d, const uint64_t* a, const uint64_t* b,
                           int64_t n, uint64_t last_mask, uint32_t* state, uint32_t* err) {
   if (n <= 0) return;
-  launch_add_kernel(stream, d, a, b, n, last_mask, state, err);
+  launch_add_kernel(stream, d, a, b, n, last_mask, state, err, false);
 }
 
 void set_add_lookback_test_hook(int64_t silent_tile, int spin_limit) {
@@ -530,7 +542,7 @@ void launch_popcount(Device& dev, const uint64_t* a, int64_t n, unsigned long lo
   int vec = aligned16(a) ? 1 : 0;
   int grid = grid_for(dev, vec ? std::max<int64_t>(n / 2, 1) : n, kThreads * (vec ? kUnroll : 1));
   ProfScope prof(dev, "k_popcount");
-  k_popcount<<<grid, kThreads, 0, dev.stream()>>>(a, n, slot, vec);
+  launch_after(dev.stream(), grid, kThreads, 0, k_popcount, a, n, slot, vec);
   check_launch();
   ++dev.n_launches;
 }
@@ -540,7 +552,7 @@ void launch_any(Device& dev, const uint64_t* a, int64_t n, unsigned int* flag) {
   const int vec = aligned16(a) ? 1 : 0;
   const int grid = grid_for(dev, vec ? std::max<int64_t>(n / 2, 1) : n, kThreads * kAnyUnroll);
   ProfScope prof(dev, "k_any");
-  k_any<<<grid, kThreads, 0, dev.stream()>>>(a, n, flag, vec);
+  launch_after(dev.stream(), grid, kThreads, 0, k_any, a, n, flag, vec);
   check_launch();
   ++dev.n_launches;
 }
@@ -549,7 +561,7 @@ void launch_fill(Device& dev, uint64_t* d, int64_t n, uint64_t value, uint64_t l
   if (n <= 0) return;
   int grid = grid_for(dev, n, kThreads * 4);
   ProfScope prof(dev, "k_fill");
-  k_fill<<<grid, kThreads, 0, dev.stream()>>>(d, n, value, last_value);
+  launch_after(dev.stream(), grid, kThreads, 0, k_fill, d, n, value, last_value);
   check_launch();
   ++dev.n_launches;
 }

@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "device.h"
+#include "pdl.cuh"
 
 namespace bsz {
 namespace {
@@ -120,6 +121,7 @@ __global__ void __launch_bounds__(kGemmWarps * 32)
 k_gemm(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C,
        const float* __restrict__ bias, const float* __restrict__ mask, float* __restrict__ colsum, int M, int N, int K,
        int relu) {
+  after_previous(A, B, bias, mask);
   extern __shared__ __align__(16) float s_mem[];
   float* As = s_mem;
   float* Bs = s_mem + kChunk * kPad;
@@ -185,6 +187,7 @@ static_assert(sizeof(float) * (kGemmWarps * kTile * kTile + kGemmWarps * kTile) 
 // loss = mean((p - t)^2), dp = 2 (p - t) / n
 __global__ void k_mse(const float* __restrict__ p, const float* __restrict__ t, float* __restrict__ dp,
                       float* __restrict__ loss, int n) {
+  after_previous(p, t);
   __shared__ float part[256];
   float s = 0.f;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -204,6 +207,7 @@ __global__ void k_mse(const float* __restrict__ p, const float* __restrict__ t, 
 __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
                        float* __restrict__ v, int64_t n, float lr, float b1, float b2, float eps,
                        float c1, float c2, float wd) {
+  after_previous(w, g, m, v);
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float gi = g[i];
@@ -223,7 +227,7 @@ template <int TA, int TB>
 void gemm(cudaStream_t s, const float* A, const float* B, float* C, const float* bias, const float* mask,
           float* colsum, int M, int N, int K, int relu) {
   dim3 grid((N + kTile - 1) / kTile, (M + kTile - 1) / kTile);
-  k_gemm<TA, TB><<<grid, kGemmWarps * 32, kGemmSmem, s>>>(A, B, C, bias, mask, colsum, M, N, K, relu);
+  launch_after(s, grid, kGemmWarps * 32, kGemmSmem, k_gemm<TA, TB>, A, B, C, bias, mask, colsum, M, N, K, relu);
   check(cudaGetLastError(), "mlp gemm launch");
 }
 
@@ -327,7 +331,7 @@ void Mlp::forward(int n) {
 
 void Mlp::backward(int n, float* loss) {
   const int L = static_cast<int>(dims_.size()) - 1;
-  k_mse<<<1, 256, 0, stream_>>>(act_[L - 1], y_, delta_[L - 1], loss_, n);
+  launch_after(stream_, 1, 256, 0, k_mse, act_[L - 1], y_, delta_[L - 1], loss_, n);
   check(cudaGetLastError(), "mlp mse");
   for (int l = L - 1; l >= 0; --l) {
     const float* in = l == 0 ? x_ : act_[l - 1];
@@ -355,9 +359,8 @@ float Mlp::train_step(const float* x, const float* y, int n, float lr) {
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, static_cast<float>(step_));
   const float c2 = 1.f - std::pow(b2, static_cast<float>(step_));
-  k_adam<<<static_cast<unsigned>((n_params_ + 255) / 256), 256, 0, stream_>>>(w_, g_, m_, v_, n_params_, lr,
-                                                                                b1, b2, 1e-8f, c1, c2,
-                                                                                weight_decay_);
+  launch_after(stream_, static_cast<unsigned>((n_params_ + 255) / 256), 256, 0, k_adam, w_, g_, m_, v_, n_params_, lr,
+               b1, b2, 1e-8f, c1, c2, weight_decay_);
   check(cudaGetLastError(), "mlp adam");
   ++launches;
   return loss;

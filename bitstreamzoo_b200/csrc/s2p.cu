@@ -17,6 +17,7 @@
 // storing 8 coalesced 256-byte rows.  Bytes past n read as zero, so every
 // stream's bits at and above n are clean.
 #include "device.h"
+#include "pdl.cuh"
 #include "s2p.h"
 
 #include <algorithm>
@@ -48,6 +49,7 @@ struct BasisOut {
 template <bool VEC, int STEPS>
 __global__ void __launch_bounds__(kS2PThreads)
 k_s2p(const uint8_t* __restrict__ bytes, int64_t n_bytes, int64_t nw, BasisOut out) {
+  after_previous(bytes);
   __shared__ uint4 s_bytes[VEC ? kS2PThreads / 32 : 1][128];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t warps = static_cast<int64_t>(gridDim.x) * (kS2PThreads / 32);
@@ -118,9 +120,9 @@ void launch_s2p(Device& dev, const uint8_t* bytes, int64_t n_bytes, uint64_t* co
   const int64_t per_block = static_cast<int64_t>(kS2PThreads) * steps;
   const unsigned blocks = static_cast<unsigned>(std::min<int64_t>((nw + per_block - 1) / per_block, 0x7fffffff));
   ProfScope prof(dev, "k_s2p");
-  if (steps == 4) k_s2p<true, 4><<<blocks, kS2PThreads, 0, dev.stream()>>>(bytes, n_bytes, nw, o);
-  else if (vec) k_s2p<true, 1><<<blocks, kS2PThreads, 0, dev.stream()>>>(bytes, n_bytes, nw, o);
-  else k_s2p<false, 1><<<blocks, kS2PThreads, 0, dev.stream()>>>(bytes, n_bytes, nw, o);
+  if (steps == 4) launch_after(dev.stream(), blocks, kS2PThreads, 0, k_s2p<true, 4>, bytes, n_bytes, nw, o);
+  else if (vec) launch_after(dev.stream(), blocks, kS2PThreads, 0, k_s2p<true, 1>, bytes, n_bytes, nw, o);
+  else launch_after(dev.stream(), blocks, kS2PThreads, 0, k_s2p<false, 1>, bytes, n_bytes, nw, o);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw CudaError(std::string("s2p launch failed: ") + cudaGetErrorString(e));
   ++dev.n_launches;
