@@ -578,9 +578,9 @@ struct Gen {
   // slots go (SlotPublish), and the code that sends them.  The CTA that
   // finishes last stores the popcounts and flags to page-locked host memory:
   // a copy after the kernel costs the stream another 5 us before the host sees
-  // them (32 Mbit program of 12 conditions: 363 us with the copies, 291 us without).  A grid of several waves
-  // leaves `publish` null and takes the copy: each CTA's fence and ticket would
-  // hold its place from the next one.
+  // them (32 Mbit program of 12 conditions: 363 us with the copies, 291 us
+  // without).  A grid of several waves leaves `publish` null and takes the
+  // copy: each CTA's fence and ticket would hold its place from the next one.
   static constexpr int kPublishFields = 4;
   static std::string publish_fields() {
     return "  u64* publish;\n  const u64* pub_from;\n  long long n_pub;\n  unsigned int* pub_done;\n";
