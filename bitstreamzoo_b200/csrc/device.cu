@@ -8,6 +8,7 @@
 #include <cstring>
 #include <exception>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -114,10 +115,22 @@ void stream_copy(char* dst, const char* src, size_t n) {
 class CopyPool {
  public:
   CopyPool(int ordinal, cudaStream_t stream) : ordinal_(ordinal), stream_(stream) {
-    BSZ_CUDA(cudaHostAlloc(&block_, kCopyRing * kCopyChunk, cudaHostAllocDefault));
-    for (cudaEvent_t& e : ev_) BSZ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     const unsigned n = std::max(1u, std::min(kCopyWorkers, std::thread::hardware_concurrency()));
-    for (unsigned i = 0; i < n; ++i) threads_.emplace_back([this] { serve(); });
+    threads_.reserve(n);
+    try {
+      BSZ_CUDA(cudaHostAlloc(&block_, kCopyRing * kCopyChunk, cudaHostAllocDefault));
+      for (cudaEvent_t& e : ev_) BSZ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      // where the process may start no more threads, those it got do
+      for (unsigned i = 0; i < n; ++i) try {
+          threads_.emplace_back([this] { serve(); });
+        } catch (const std::system_error&) {
+          if (threads_.empty()) throw;
+          break;
+        }
+    } catch (...) {
+      release();
+      throw;
+    }
   }
   ~CopyPool() {
     {
@@ -126,9 +139,7 @@ class CopyPool {
     }
     wake_.notify_all();
     for (auto& t : threads_) t.join();
-    for (cudaEvent_t e : ev_)
-      if (e) cudaEventDestroy(e);
-    if (block_) cudaFreeHost(block_);
+    release();
   }
   CopyPool(const CopyPool&) = delete;
   CopyPool& operator=(const CopyPool&) = delete;
@@ -196,6 +207,12 @@ class CopyPool {
   std::atomic<size_t> next_{0}, issued_{0};
   std::atomic<size_t> copied_[kCopyRing] = {};   // memcpys done with each buffer in this job
   std::atomic<bool> failed_{false};
+
+  void release() {
+    for (cudaEvent_t e : ev_)
+      if (e) cudaEventDestroy(e);
+    if (block_) cudaFreeHost(block_);
+  }
 
   char* buffer(size_t b) const { return static_cast<char*>(block_) + b * kCopyChunk; }
 
