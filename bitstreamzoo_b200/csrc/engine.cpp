@@ -783,17 +783,21 @@ void Executor::flush(const Bits* live, int* extra) {
     if (pending(i)) seg.order.push_back(i);
     else seg.inputs.push_back(i);
   }
-  for (auto& p : pending_pops_) seg.pops.push_back({p.first, p.second - slot_base_});
-  // this segment's popcount slots (allocated consecutively since the last
-  // flush) start at zero: the kernels accumulate into them
+  // This segment's popcount slots (allocated consecutively since the last
+  // flush) start at zero: the kernels accumulate into them.  They are numbered
+  // from the segment's first one: a generated kernel holds these numbers, and
+  // the same loop body has to be the same kernel in every trip (a new one per
+  // trip costs its compilation, 80 ms and more).
   int64_t pop_lo = 0, n_pops = 0;
-  if (!seg.pops.empty()) {
-    int64_t hi = pop_lo = seg.pops.front().second;
-    for (auto& p : seg.pops) {
-      pop_lo = std::min(pop_lo, p.second);
+  if (!pending_pops_.empty()) {
+    int64_t lo = pending_pops_.front().second, hi = lo;
+    for (auto& p : pending_pops_) {
+      lo = std::min(lo, p.second);
       hi = std::max(hi, p.second);
     }
-    n_pops = hi - pop_lo + 1;
+    pop_lo = lo - slot_base_;
+    n_pops = hi - lo + 1;
+    for (auto& p : pending_pops_) seg.pops.push_back({p.first, p.second - lo});
   }
   t_segment_ms += ms_since(t0);
   if (!seg.order.empty() || !seg.pops.empty()) {
@@ -850,14 +854,14 @@ void Executor::flush(const Bits* live, int* extra) {
         pub.n = n_pub;
         pub.done = reinterpret_cast<unsigned int*>(d_slots_ + at + flag_words - 1);
       }
-      if (fused_->run(nodes_, seg, N_, nw_, d_slots_, reinterpret_cast<unsigned int*>(d_slots_ + at), pub)) {
+      if (fused_->run(nodes_, seg, N_, nw_, d_slots_ + pop_lo, reinterpret_cast<unsigned int*>(d_slots_ + at), pub)) {
         published_ = pub_buf_;
         published_from_ = resolved_upto_;
         published_count_ = n_pub;
       }
     } else {
       zero_slots(pop_lo, n_pops);
-      run_plain(seg);
+      run_plain(seg, d_slots_ + pop_lo);
     }
     t_run_ms += ms_since(t2);
   }
@@ -893,7 +897,7 @@ const uint64_t* Executor::const_ptr(int node) {
   return (*slot)->p;
 }
 
-void Executor::run_plain(const Segment& seg) {
+void Executor::run_plain(const Segment& seg, unsigned long long* slots) {
   const int n_nodes = static_cast<int>(nodes_.size());
   std::vector<int> uses(n_nodes, 0);
   std::vector<uint8_t> keep(n_nodes, 0);
@@ -907,7 +911,7 @@ void Executor::run_plain(const Segment& seg) {
   }
   auto launch_pops = [&](int id) {
     for (int64_t slot : pops_of[id])
-      launch_popcount(dev_, nodes_[id].buf ? nodes_[id].buf->p : const_ptr(id), nw_, d_slots_ + slot);
+      launch_popcount(dev_, nodes_[id].buf ? nodes_[id].buf->p : const_ptr(id), nw_, slots + slot);
   };
   for (int i : seg.inputs) launch_pops(i);
   for (int id : seg.order) {
@@ -1071,7 +1075,7 @@ void Executor::run_vm(const Segment& seg, int64_t pop_lo, int64_t n_pops) {
         VmOp op{};
         op.code = kVmPop;
         op.a = loc[node];
-        op.dst = static_cast<int32_t>(it->second - pop_lo);
+        op.dst = static_cast<int32_t>(it->second);
         ops.push_back(op);
       }
     };

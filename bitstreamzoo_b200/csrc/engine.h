@@ -272,7 +272,7 @@ class Executor {
   bool pending(int node) const;
   void flush(const std::vector<uint64_t>* live, int* extra);
   void compact(int* extra);
-  void run_plain(const Segment& seg);
+  void run_plain(const Segment& seg, unsigned long long* slots);
   // pop_lo, n_pops: the popcount slots that the segment accumulates into.
   void run_vm(const Segment& seg, int64_t pop_lo, int64_t n_pops);
   // Whole program, control flow included, as one device-interpreter launch
