@@ -460,6 +460,7 @@ int Executor::rhs(const SExpr& e) {
     }
     case SExpr::Bin: {
       int a = operand(*e.a);
+      Held keep(*this, &a);   // the other operand's index may need a flush
       int b = operand(*e.b);
       NOp op = e.op == '&' ? NOp::And : e.op == '|' ? NOp::Or : e.op == '^' ? NOp::Xor : NOp::Add;
       const char* name = e.op == '&' ? "&" : e.op == '|' ? "|" : e.op == '^' ? "^" : "+";
@@ -468,6 +469,7 @@ int Executor::rhs(const SExpr& e) {
     }
     case SExpr::Shift: {
       int a = operand(*e.a);
+      Held keep(*this, &a);
       int64_t k = force(ival(*e.index));
       if (k < 0) throw RuntimeError("negative shift count");
       count(e.op == '<' ? "<<" : ">>");
@@ -512,6 +514,7 @@ Executor::IntV Executor::popcount(int node) {
   count("popcount");
   if (n.op == NOp::Zero) return IntV{0, -1};
   if (n.op == NOp::OnesMask && !tracing_) return IntV{N_, -1};
+  Held keep(*this, &node);
   if (!tracing_) ensure_slots(1);
   int64_t slot = n_slots_++;
   pending_pops_.push_back({node, slot});
@@ -541,24 +544,26 @@ bool Executor::nonzero(int node, const Stmt* at) {
   if (n.tail) return true;                // negative value: nonzero
   if (n.op == NOp::Zero) return false;
   if (n.op == NOp::OnesMask || n.op == NOp::AllOnes) return N_ > 0;
-  int x = node;
+  Held keep(*this, &node);
   auto it = at ? live_->at.find(at->id) : live_->at.end();
+  const Bits* live = it == live_->at.end() ? nullptr : &it->second;
+  const bool counted = pending(node) && opt_.mode != ExecMode::Plain;
+  if (counted) ensure_slots(1);   // may compute the value
   // A value still to be computed is counted by the segment that computes it:
   // its count, the other popcounts and the speculation flags come back in one
   // copy, with no pass over the value of its own.
-  if (pending(node) && opt_.mode != ExecMode::Plain) {
-    ensure_slots(1);
+  if (counted && pending(node)) {
     const int64_t slot = n_slots_++;
     pending_pops_.push_back({node, slot});
-    flush(it == live_->at.end() ? nullptr : &it->second, &x);
+    flush(live);
     settle();
     check_error();
     return slot_val_[slot] != 0;
   }
-  flush(it == live_->at.end() ? nullptr : &it->second, &x);
+  flush(live);
   if (fused_ && fused_->pending()) settle();   // the condition reads the segment's output
   BSZ_CUDA(cudaMemsetAsync(d_flag_, 0, 4, dev_.stream()));
-  launch_any(dev_, nodes_[x].buf->p, nw_, d_flag_);
+  launch_any(dev_, nodes_[node].buf->p, nw_, d_flag_);
   unsigned int h = 0;
   BSZ_CUDA(cudaMemcpyAsync(&h, d_flag_, 4, cudaMemcpyDeviceToHost, dev_.stream()));
   dev_.sync();
@@ -570,7 +575,7 @@ bool Executor::nonzero(int node, const Stmt* at) {
 void Executor::exec_block(const std::vector<Stmt>& v) {
   for (const auto& s : v) {
     exec(s);
-    if (!tracing_ && nodes_.size() > nodes_after_flush_ + kAutoFlushNodes) flush(nullptr, nullptr);
+    if (!tracing_ && nodes_.size() > nodes_after_flush_ + kAutoFlushNodes) flush(nullptr);
   }
 }
 
@@ -665,7 +670,7 @@ void Executor::run(bool finish_now) {
     if (straight && n_flushes_ == f0) save_walk(key, n0);
   }
   final_flush_ = true;
-  flush(&live_->end, nullptr);
+  flush(&live_->end);
   final_flush_ = false;
   publish_op_mix();
   // Outputs bound to constants get a buffer so the caller can read them.
@@ -736,7 +741,7 @@ void Executor::finish() {
 
 // ----------------------------------------------------------------- flush ---
 
-void Executor::flush(const Bits* live, int* extra) {
+void Executor::flush(const Bits* live) {
   if (tracing_)
     throw RuntimeError("batch execution needs straight-line programs: this one needs the device "
                        "during the walk (a stream condition, or a popcount used as a loop bound, "
@@ -765,7 +770,7 @@ void Executor::flush(const Bits* live, int* extra) {
   }
   for (auto& a : arrs_)
     if (a) for (auto& kv : a->elems) add_target(kv.second);
-  if (extra) add_target(*extra);
+  for (int* h : held_) add_target(*h);
   std::vector<int> stack(seg.outputs.begin(), seg.outputs.end());
   for (auto& p : pending_pops_) stack.push_back(p.first);
   while (!stack.empty()) {
@@ -868,7 +873,7 @@ void Executor::flush(const Bits* live, int* extra) {
   auto t3 = clk::now();
   pending_pops_.clear();
   max_live_buffers = std::max(max_live_buffers, live_buffer_count());
-  compact(extra);
+  compact();
   t_compact_ms += ms_since(t3);
 }
 
@@ -1224,7 +1229,7 @@ void Executor::run_vm(const Segment& seg, int64_t pop_lo, int64_t n_pops) {
   max_live_buffers = std::max(max_live_buffers, live_buffer_count() + n_slots);
 }
 
-void Executor::compact(int* extra) {
+void Executor::compact() {
   std::vector<Node> old;
   old.swap(nodes_);
   cse_.clear();
@@ -1251,7 +1256,7 @@ void Executor::compact(int* extra) {
   for (auto& v : var_) v = map(v);
   for (auto& a : arrs_)
     if (a) for (auto& kv : a->elems) kv.second = map(kv.second);
-  if (extra) *extra = map(*extra);
+  for (int* h : held_) *h = map(*h);
   nodes_after_flush_ = nodes_.size();
   if (fused_ && fused_->pending()) fused_->keep_nodes(std::move(old));
 }
@@ -1274,7 +1279,7 @@ void Executor::ensure_slots(int64_t need) {
 }
 
 void Executor::resolve_slots() {
-  if (!pending_pops_.empty()) flush(nullptr, nullptr);
+  if (!pending_pops_.empty()) flush(nullptr);
   settle();
 }
 

@@ -270,8 +270,19 @@ class Executor {
   int mk_raw(NOp op, int a, int b, int64_t k, uint8_t tail);
   int buf_node(BufRef buf, uint8_t tail, bool clean);
   bool pending(int node) const;
-  void flush(const std::vector<uint64_t>* live, int* extra);
-  void compact(int* extra);
+  // Computes what is pending and live.  Every node is renumbered: a node id
+  // kept in a local variable across anything that may flush (a slot taken, an
+  // int read, a condition) has to be Held meanwhile.
+  void flush(const std::vector<uint64_t>* live);
+  void compact();
+  struct Held {
+    Executor& ex;
+    Held(Executor& e, int* node) : ex(e) { ex.held_.push_back(node); }
+    ~Held() { ex.held_.pop_back(); }
+    Held(const Held&) = delete;
+    Held& operator=(const Held&) = delete;
+  };
+  std::vector<int*> held_;
   void run_plain(const Segment& seg, unsigned long long* slots);
   // pop_lo, n_pops: the popcount slots that the segment accumulates into.
   void run_vm(const Segment& seg, int64_t pop_lo, int64_t n_pops);
