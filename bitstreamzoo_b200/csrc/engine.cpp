@@ -835,6 +835,13 @@ void Executor::flush(const Bits* live) {
       // (and the counter of the CTAs that are done, for the copy to the host).
       const int64_t flag_words = (fused_->prepare(nodes_, seg, N_, nw_, &compile_ms) + 1) / 2 + 1;
       if (slot_cap_ == 0) ensure_slots(0);
+      // A segment with popcounts finds room behind them (ensure_slots leaves
+      // it); one without may be the last of many that took flags only.
+      if (n_pops == 0 && n_slots_ - slot_base_ + flag_words > slot_cap_) {
+        settle();
+        slot_base_ = n_slots_;
+        zeroed_ = 0;
+      }
       flags_slot_ = n_slots_;
       const int64_t at = n_slots_ - slot_base_;
       if (at + flag_words > slot_cap_ + kFlagSlots) throw RuntimeError("internal: no room for the parts' flags");

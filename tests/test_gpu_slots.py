@@ -70,3 +70,17 @@ def test_operands_across_an_int_that_has_to_be_read(ctx, mode):
     r = ctx.run(src, nbits, inputs, mode=mode)
     for name in "xyw":
         assert r.stream_int(name) == want[name] & ((1 << nbits) - 1), name
+
+
+def test_more_segments_without_popcounts_than_a_chunk_has_slots(ctx):
+    """A condition on an input takes no slot, the segment computed for it two."""
+    trips, words = 35_500, 600
+    rng = np.random.default_rng(3)
+    a, b = wl.random_words(rng, 64 * words), wl.random_words(rng, 64 * words)
+    src = ("input stream a\ninput stream b\ninput stream m\noutput stream acc\noutput int n\nn = 0\nacc = b\n"
+           "int trips = popcount(m)\nfor i in 0..trips {\n  stream t = acc ^ a\n  acc = t\n"
+           "  if (a) {\n    n = n + 1\n  }\n}\n")
+    r = ctx.run(src, 64 * words, {"a": a, "b": b, "m": _bits(trips, words)}, mode=bz.MODE_FUSED)
+    assert r.int("n") == trips
+    assert np.array_equal(r.stream("acc"), b if trips % 2 == 0 else a ^ b)
+    assert r.stats["n_fused_launches"] >= trips
