@@ -623,19 +623,25 @@ struct Gen {
     body(s);
     s << "  }\n";
     if (!part.pops.empty()) {
-      // one atomic per CTA and popcount: with one per warp, 2^14 warps of a
-      // 2^32-bit program spent as long on their atomics as on their words
-      s << "  __shared__ unsigned long long s_pc[" << warps << "][" << part.pops.size() << "];\n"
+      // One atomic per CTA and popcount: with one per warp, 2^14 warps of a
+      // 2^32-bit program spent as long on their atomics as on their words.
+      // In rounds of as many popcounts as 16 KiB of shared memory hold.
+      const size_t round = std::min<size_t>(part.pops.size(), 2048 / static_cast<size_t>(warps));
+      s << "  __shared__ unsigned long long s_pc[" << warps << "][" << round << "];\n"
         << "  const int warp = threadIdx.x >> 5;\n";
-      for (size_t j = 0; j < part.pops.size(); ++j)
-        s << "  {\n    unsigned long long t = pc" << j << ";\n"
-          << "    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(~0u, t, o);\n"
-          << "    if (lane == 0) s_pc[warp][" << j << "] = t;\n  }\n";
-      s << "  __syncthreads();\n";
-      for (size_t j = 0; j < part.pops.size(); ++j)
-        s << "  if (threadIdx.x == " << j % (static_cast<size_t>(warps) * 32) << ") {\n    unsigned long long t = 0;\n    for (int k = 0; k < " << warps
-          << "; ++k) t += s_pc[k][" << j << "];\n    if (t) atomicAdd(A.slots + " << part.pops[j].second
-          << ", t);\n  }\n";
+      for (size_t first = 0; first < part.pops.size(); first += round) {
+        const size_t end = std::min(part.pops.size(), first + round);
+        if (first) s << "  __syncthreads();\n";
+        for (size_t j = first; j < end; ++j)
+          s << "  {\n    unsigned long long t = pc" << j << ";\n"
+            << "    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(~0u, t, o);\n"
+            << "    if (lane == 0) s_pc[warp][" << j - first << "] = t;\n  }\n";
+        s << "  __syncthreads();\n";
+        for (size_t j = first; j < end; ++j)
+          s << "  if (threadIdx.x == " << j % (static_cast<size_t>(warps) * 32)
+            << ") {\n    unsigned long long t = 0;\n    for (int k = 0; k < " << warps << "; ++k) t += s_pc[k]["
+            << j - first << "];\n    if (t) atomicAdd(A.slots + " << part.pops[j].second << ", t);\n  }\n";
+      }
     }
     s << publish_tail() << "}\n";
     return s.str();
