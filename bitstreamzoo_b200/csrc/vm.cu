@@ -827,6 +827,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
           if (m.ctas * m.warps > 1) {
             const uint4 q = reinterpret_cast<const uint4*>(m.exchange(c))[m.lane];
             c = __reduce_add_sync(0xffffffffu, q.x + q.y + q.z + q.w);
+          } else {
+            __syncwarp();   // a barrier for the shifts behind it (vm_finish)
           }
           iregs[dst] = static_cast<long long>(c);
           break;
