@@ -698,6 +698,13 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
       }
   }
   m.barrier();   // exchange tables cleared everywhere, inputs loaded
+  // A value of the warp's own that its lanes share: all have read what it was
+  // computed from before one of them writes it, and see it from then on.
+  auto set_shared = [&](auto* p, auto v) {
+    __syncwarp();
+    if (m.lane == 0) *p = v;
+    __syncwarp();
+  };
   uint32_t err = kVmOk;
   int64_t executed = 0;
   int i = static_cast<int>(X.n_loads);
@@ -718,7 +725,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
       if (o.x & (kVmBar << 16)) m.barrier();
       const bool track = PROG && (o.x & (kVmTrack << 16));
       const bool keep = o.x & (kVmKeepA << 16), keep_out = !(o.x & (kVmNoStore << 16));
-      auto tail = [&](int v) -> uint8_t& { return tails[v / X.unit]; };
+      auto tail = [&](int v) -> uint32_t { return tails[v / X.unit]; };
+      auto set_tail = [&](int v, uint32_t t) { set_shared(tails + v / X.unit, static_cast<uint8_t>(t)); };
+      auto set_int = [&](int r, long long v) { set_shared(iregs + r, v); };
       uint64_t y[4];
       if (code <= kVmAndNot) {   // the commonest first
         if (!keep) m.load(x, a);
@@ -741,8 +750,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
         }
         if (keep_out) m.store(x, dst);
         if (track)
-          tail(dst) = code == kVmAnd ? tail(a) & tail(b) : code == kVmOr ? tail(a) | tail(b)
-                      : code == kVmXor ? tail(a) ^ tail(b) : 0;
+          set_tail(dst, code == kVmAnd ? tail(a) & tail(b) : code == kVmOr ? tail(a) | tail(b)
+                        : code == kVmXor ? tail(a) ^ tail(b) : 0);
         continue;
       }
       if (code == kVmAdd) {
@@ -750,14 +759,14 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
         m.load(y, b);
         m.add(x, y);
         if (keep_out) m.store(x, dst);
-        if (track) tail(dst) = 0;
+        if (track) set_tail(dst, 0);
         continue;
       }
       if (code == kVmShl) {
         if (!keep) m.load(x, a);
         m.shl(x, a, b);
         if (keep_out) m.store(x, dst);
-        if (track) tail(dst) = 0;
+        if (track) set_tail(dst, 0);
         continue;
       }
       switch (code) {
@@ -766,7 +775,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
           if (!keep) m.load(x, a);
           m.shr(x, a, b, t ? ~uint64_t(0) : 0);
           if (keep_out) m.store(x, dst);
-          if (track) tail(dst) = static_cast<uint8_t>(t);
+          if (track) set_tail(dst, static_cast<uint8_t>(t));
           break;
         }
         case kVmPop: {
@@ -778,20 +787,20 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
         case kVmCopy:
           if (!keep) m.load(x, a);
           if (keep_out) m.store(x, dst);
-          if (track) tail(dst) = tail(a);
+          if (track) set_tail(dst, tail(a));
           break;
         case kVmFill: {
           const uint32_t f = (o.x >> 8) & 0xff;
 #pragma unroll
           for (int j = 0; j < 4; ++j) x[j] = f == 0 || m.w0 + j >= m.nw ? 0 : f == 1 ? m.lm[j] : ~uint64_t(0);
           m.store(x, dst);
-          if (track) tail(dst) = f == 2 ? 1 : 0;
+          if (track) set_tail(dst, f == 2 ? 1 : 0);
           break;
         }
         case kVmLoad:   // inputs past the first kVmWindow
           m.load_ext(x, op_pointer(a, b));
           m.store(x, dst);
-          if (track) tail(dst) = (o.x >> 8) & 0xff;
+          if (track) set_tail(dst, (o.x >> 8) & 0xff);
           break;
         case kVmStore:
           if (!keep) m.load(x, a);
@@ -830,31 +839,31 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
           } else {
             __syncwarp();   // a barrier for the shifts behind it (vm_finish)
           }
-          iregs[dst] = static_cast<long long>(c);
+          set_int(dst, static_cast<long long>(c));
           break;
         }
         case kVmIConst:
-          if (PROG) iregs[dst] = static_cast<long long>(reinterpret_cast<uintptr_t>(op_pointer(a, b)));
+          if (PROG) set_int(dst, static_cast<long long>(reinterpret_cast<uintptr_t>(op_pointer(a, b))));
           break;
         // two's-complement wrap, like the int64 host arithmetic
         case kVmIAdd:
-          if (PROG) iregs[dst] = static_cast<long long>(static_cast<uint64_t>(iregs[a]) + static_cast<uint64_t>(iregs[b]));
+          if (PROG) set_int(dst, static_cast<long long>(static_cast<uint64_t>(iregs[a]) + static_cast<uint64_t>(iregs[b])));
           break;
         case kVmISub:
-          if (PROG) iregs[dst] = static_cast<long long>(static_cast<uint64_t>(iregs[a]) - static_cast<uint64_t>(iregs[b]));
+          if (PROG) set_int(dst, static_cast<long long>(static_cast<uint64_t>(iregs[a]) - static_cast<uint64_t>(iregs[b])));
           break;
         case kVmIMul:
-          if (PROG) iregs[dst] = static_cast<long long>(static_cast<uint64_t>(iregs[a]) * static_cast<uint64_t>(iregs[b]));
+          if (PROG) set_int(dst, static_cast<long long>(static_cast<uint64_t>(iregs[a]) * static_cast<uint64_t>(iregs[b])));
           break;
         case kVmTick: {
           if (!PROG) break;
           const long long t = iregs[dst] + 1;
-          iregs[dst] = t;
+          set_int(dst, t);
           if (t > 10000) err = kVmErrWhile;
           break;
         }
         case kVmInc:
-          if (PROG) iregs[dst] += 1;
+          if (PROG) set_int(dst, iregs[dst] + 1);
           break;
         case kVmErr:
           if (PROG) err = static_cast<uint32_t>(a);

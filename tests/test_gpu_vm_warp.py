@@ -1,6 +1,6 @@
 """Programs that the device interpreter runs in one warp (streams of up to 128
 words), where lanes share words without a barrier of several warps between
-them: a shift behind a popcount."""
+them: a shift behind a popcount, ints that are their own operands."""
 
 import numpy as np
 import pytest
@@ -33,9 +33,42 @@ while (pend) {
 }
 """
 
+INTS = """input stream a
+input stream b
+output int n
+output int m
+output int k
+output stream acc
+stream z = a ^ b
+n = popcount(z)
+n = n + n
+n = n * n
+m = 0
+k = 5
+acc = b
+stream pend = a
+while (pend) {
+  stream x = acc & pend
+  int c = popcount(x)
+  n = c - n
+  m = m + c
+  m = m * c
+  k = k - m
+  if (x) {
+    k = c + k
+    stream y = acc ^ pend
+    acc = y
+  }
+  stream p = pend << 61
+  pend = p
+}
+k = k - n
+"""
+
+
 @pytest.mark.parametrize("words", [1, 4, 5, 33, 127, 128])
-def test_shift_after_a_count(ctx, words):
-    src = SHIFT_AFTER_COUNT
+@pytest.mark.parametrize("src", [SHIFT_AFTER_COUNT, INTS], ids=["shift", "ints"])
+def test_one_warp(ctx, words, src):
     nbits = 64 * words - 3
     rng = np.random.default_rng(words)
     a = wl.random_words(rng, nbits)
@@ -46,5 +79,6 @@ def test_shift_after_a_count(ctx, words):
         got = ctx.run(src, nbits, inputs, mode=bz.MODE_VM)
         assert got.stats["n_vm_launches"] == 1
         assert np.array_equal(got.stream("acc"), want.stream("acc"))
-        assert got.int("n") == want.int("n")
+        for name in ("n", "m", "k")[:1 if src is SHIFT_AFTER_COUNT else 3]:
+            assert got.int(name) == want.int(name), name
         assert got.stats["op_count"] == want.stats["op_count"]
