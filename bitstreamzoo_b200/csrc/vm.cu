@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
     __syncwarp();
   };
   uint32_t err = kVmOk;
-  int64_t executed = 0;
+  int64_t executed = 0;    // beyond one pass over the list: jumps back, less what jumps ahead skip
   int i = static_cast<int>(X.n_loads);
   uint64_t x[4] = {0, 0, 0, 0};   // the last instruction's value stays here (kVmKeepA)
   while (true) {
@@ -816,10 +816,13 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
           } else {
             __syncwarp();
           }
-          if (!any && !((o.x & (kVmTailA << 16)) && tail(a))) jump = b;
+          if (!any && !((o.x & (kVmTailA << 16)) && tail(a))) {
+            executed -= b - (first + i);   // skipped
+            jump = b;
+          }
           break;
         }
-        case kVmJmp:   // to a loop's condition: its body has run
+        case kVmJmp:   // back to a loop's condition
           if (!PROG) break;
           executed += first + i - b;
           if (executed > kVmMaxExecuted) err = kVmErrBudget;
