@@ -966,7 +966,7 @@ bool Executor::fused_pays(const Segment& seg) {
   const double per_op_ms = 0.004 + 24.0 * static_cast<double>(nw_) / 6.5e9;
   const double compile_ms_est = 60.0 + 0.4 * static_cast<double>(seg.order.size());
   if (ops * per_op_ms > compile_ms_est) return true;
-  return fused_->all_compiled(nodes_, seg, N_);
+  return fused_->all_compiled(nodes_, seg, N_, nw_);
 }
 
 void Executor::run_vm(const Segment& seg, int64_t pop_lo, int64_t n_pops) {

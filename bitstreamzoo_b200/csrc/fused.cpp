@@ -1758,61 +1758,69 @@ std::unordered_map<std::string, std::shared_ptr<const SegPlan>>& plan_cache() {
   return m;
 }
 
-PartKernel part_kernel(const std::vector<Node>& nodes, const Part& p, int64_t N, const Schedule& sc,
+// The source of a part's kernel and what its launch needs of the generator.
+// `sc` becomes the schedule that the part takes: the register form where the
+// TMA form's argument block (a 128-byte tensor map per read input and per
+// output, 24 at most) or its boxes in one SM's shared memory would not fit.
+std::string part_source(const std::vector<Node>& nodes, const Part& p, int64_t N, Schedule& sc, PartKernel& pk) {
+  const bool masked = (N % 64) != 0;
+  if (sc.layout == 2) {
+    int n_maps = static_cast<int>(p.outputs.size());
+    for (int n : p.inputs)
+      if (!is_const(nodes[n].op)) ++n_maps;
+    if (n_maps <= 24) {
+      GenSeq g{nodes, p, N, sc.warps, 1, masked};
+      g.tma = true;
+      g.roww = sc.chunk_words == 4 ? 4 : 8;
+      g.stages = sc.stages == 3 ? 3 : 2;
+      g.unroll_pairs = sc.unroll != 0;
+      g.shift_mul = sc.shift_mul != 0;
+      std::string src = g.source();
+      if (g.smem_bytes() <= 227 * 1024) {
+        pk.warm = g.warm;
+        pk.roww = g.roww;
+        pk.smem = g.smem_bytes();
+        pk.mapped = g.mapped;
+        return src;
+      }
+    }
+    sc.layout = 1;
+    sc.min_blocks = 1;
+  }
+  if (sc.layout == 1) {
+    GenSeq g{nodes, p, N, sc.warps, sc.min_blocks, masked};
+    g.shift_mul = sc.shift_mul != 0;
+    g.reg_chunk = sc.chunk_words == 8 ? 8 : 4;
+    std::string src = g.source();
+    pk.warm = g.warm;
+    return src;
+  }
+  Gen g{nodes, p, N, sc.warps, sc.min_blocks, masked, sc.prefetch != 0};
+  std::string src = g.source();
+  pk.warm = g.warm;
+  pk.blocked = g.block_steps() > 1;
+  return src;
+}
+
+PartKernel part_kernel(const std::vector<Node>& nodes, const Part& p, int64_t N, const Schedule& sched,
                        double* compile_ms) {
-  const std::string key = part_key(nodes, p, (N % 64) != 0, sc);
+  const std::string key = part_key(nodes, p, (N % 64) != 0, sched);
   {
     std::lock_guard<std::mutex> lk(g_part_mu);
     auto it = part_cache().find(key);
     if (it != part_cache().end()) return it->second;
   }
   PartKernel pk;
-  // the TMA form's argument block holds a 128-byte tensor map per read input
-  // and per output; past 24 of them the part takes the register form
-  int n_maps = static_cast<int>(p.outputs.size());
-  for (int n : p.inputs)
-    if (!is_const(nodes[n].op)) ++n_maps;
-  if (sc.layout == 2 && n_maps > 24) {
-    Schedule s1 = sc;
-    s1.layout = 1;
-    s1.min_blocks = 1;
-    return part_kernel(nodes, p, N, s1, compile_ms);
-  }
-  if (sc.layout == 2) {
-    GenSeq g{nodes, p, N, sc.warps, 1, (N % 64) != 0};
-    g.tma = true;
-    g.roww = sc.chunk_words == 4 ? 4 : 8;
-    g.stages = sc.stages == 3 ? 3 : 2;
-    g.unroll_pairs = sc.unroll != 0;
-    g.shift_mul = sc.shift_mul != 0;
-    const std::string src = g.source();
-    pk.c = compile_source(src, sc.warps * 32, compile_ms);
-    pk.warm = g.warm;
-    pk.roww = g.roww;
-    pk.smem = g.smem_bytes();
-    pk.mapped = g.mapped;
-    if (pk.smem > 227 * 1024 ||
-        drv().func_set_attribute(pk.c.fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, pk.smem) != CUDA_SUCCESS ||
-        drv().occupancy(&pk.tma_blocks_per_sm, pk.c.fn, sc.warps * 32, pk.smem) != CUDA_SUCCESS ||
-        pk.tma_blocks_per_sm < 1) {
-      // the boxes of this part do not fit in one SM's shared memory at this
-      // CTA size: the part takes the register form
-      Schedule s1 = sc;
-      s1.layout = 1;
-      s1.min_blocks = 1;
-      return part_kernel(nodes, p, N, s1, compile_ms);
-    }
-  } else if (sc.layout == 1) {
-    GenSeq g{nodes, p, N, sc.warps, sc.min_blocks, (N % 64) != 0};
-    g.shift_mul = sc.shift_mul != 0;
-    g.reg_chunk = sc.chunk_words == 8 ? 8 : 4;
-    pk.c = compile_source(g.source(), sc.warps * 32, compile_ms);
-    pk.warm = g.warm;
-  } else {
-    Gen g{nodes, p, N, sc.warps, sc.min_blocks, (N % 64) != 0, sc.prefetch != 0};
-    pk.c = compile_source(g.source(), sc.warps * 32, compile_ms);
-    pk.warm = g.warm;
-    pk.blocked = g.block_steps() > 1;
+  Schedule sc = sched;
+  pk.c = compile_source(part_source(nodes, p, N, sc, pk), sc.warps * 32, compile_ms);
+  if (pk.roww > 0 &&
+      (drv().func_set_attribute(pk.c.fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, pk.smem) != CUDA_SUCCESS ||
+       drv().occupancy(&pk.tma_blocks_per_sm, pk.c.fn, sc.warps * 32, pk.smem) != CUDA_SUCCESS ||
+       pk.tma_blocks_per_sm < 1)) {
+    // no CTA of this size fits an SM with its boxes: the register form
+    sc.layout = 1;
+    sc.min_blocks = 1;
+    return part_kernel(nodes, p, N, sc, compile_ms);
   }
   std::lock_guard<std::mutex> lk(g_part_mu);
   part_cache()[key] = pk;
@@ -1953,74 +1961,69 @@ Schedule pick_form(const std::vector<Node>& nodes, const Segment& seg, int64_t n
 
 }  // namespace
 
-bool FusedBackend::all_compiled(const std::vector<Node>& nodes, const Segment& seg, int64_t N) {
-  const Schedule sc = impl_->scheduled ? impl_->opt.sched : pick_form(nodes, seg, (N + 63) / 64);
-  {
-    std::lock_guard<std::mutex> lk(g_plan_mu);
-    if (plan_cache().count(graph_key(nodes, seg.order, seg.inputs, seg.outputs, seg.pops, (N % 64) != 0, sc)))
-      return true;
-  }
-  std::vector<Part> parts = split(nodes, seg, sc.cut_adds, sc.layout >= 1 ? 1 : 32);
-  for (Part& p : parts) {
-    if ((p.order.empty() && p.pops.empty()) || p.lookback_add) continue;
-    if (p.inputs.size() > kMaxInputs) return false;
-    {
-      std::lock_guard<std::mutex> lk(g_part_mu);
-      if (part_cache().count(part_key(nodes, p, (N % 64) != 0, sc))) continue;
-    }
-    if (sc.layout == 2) {
-      GenSeq g{nodes, p, N, sc.warps, 1, (N % 64) != 0};
-      g.tma = true;
-      g.roww = sc.chunk_words == 4 ? 4 : 8;
-      g.stages = sc.stages == 3 ? 3 : 2;
-      g.unroll_pairs = sc.unroll != 0;
-      g.shift_mul = sc.shift_mul != 0;
-      if (!is_compiled(g.source())) return false;
-    } else if (sc.layout == 1) {
-      GenSeq g{nodes, p, N, sc.warps, sc.min_blocks, (N % 64) != 0};
-      g.shift_mul = sc.shift_mul != 0;
-      g.reg_chunk = sc.chunk_words == 8 ? 8 : 4;
-      if (!is_compiled(g.source())) return false;
-    } else {
-      Gen g{nodes, p, N, sc.warps, sc.min_blocks, (N % 64) != 0, sc.prefetch != 0};
-      if (!is_compiled(g.source())) return false;
-    }
-  }
-  return true;
-}
-
-
-int64_t FusedBackend::prepare(const std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
-                              double* compile_ms) {
-  Schedule sc = impl_->scheduled ? impl_->opt.sched : pick_form(nodes, seg, nw);
-  if (sc.layout >= 1) {
+// The schedule that a segment runs with.
+FusedBackend::Choice FusedBackend::choose(const std::vector<Node>& nodes, const Segment& seg, int64_t N,
+                                          int64_t nw) const {
+  Choice c;
+  c.sched = impl_->scheduled ? impl_->opt.sched : pick_form(nodes, seg, nw);
+  if (c.sched.layout >= 1) {
     // the thread-sequential forms move 32-byte sectors: every input must be
     // 32-byte aligned (the library's own buffers are 256-byte aligned; a
     // borrowed caller buffer may not be), else the segment takes the warp form
     for (int n : seg.inputs)
-      if (nodes[n].buf && (reinterpret_cast<uintptr_t>(nodes[n].buf->p) & 31)) sc.layout = 0;
+      if (nodes[n].buf && (reinterpret_cast<uintptr_t>(nodes[n].buf->p) & 31)) c.sched.layout = 0;
   }
   // the TMA form pays off on long streams only (its boxes cover 32 threads'
   // ranges); short ones take the register form
-  if (sc.layout == 2 && nw < (int64_t(1) << 16)) sc.layout = 1;
-  using clk = std::chrono::steady_clock;
-  auto ms_since = [](clk::time_point t) { return std::chrono::duration<double, std::milli>(clk::now() - t).count(); };
-  auto tp = clk::now();
-  std::string skey = graph_key(nodes, seg.order, seg.inputs, seg.outputs, seg.pops, (N % 64) != 0, sc);
-  std::string spec_key;
-  if (sc.cut_adds == 0) {
+  if (c.sched.layout == 2 && nw < (int64_t(1) << 16)) c.sched.layout = 1;
+  auto key = [&] {
+    return graph_key(nodes, seg.order, seg.inputs, seg.outputs, seg.pops, (N % 64) != 0, c.sched);
+  };
+  c.key = key();
+  if (c.sched.cut_adds == 0) {
     bool failed_before;
     {
       std::lock_guard<std::mutex> lk(g_spec_mu);
-      failed_before = spec_failed().count(skey) != 0;
+      failed_before = spec_failed().count(c.key) != 0;
     }
     if (failed_before) {
-      sc.cut_adds = 2;
-      skey = graph_key(nodes, seg.order, seg.inputs, seg.outputs, seg.pops, (N % 64) != 0, sc);
+      c.sched.cut_adds = 2;
+      c.key = key();
     } else {
-      spec_key = skey;
+      c.spec_key = c.key;
     }
   }
+  return c;
+}
+
+bool FusedBackend::all_compiled(const std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw) {
+  const Choice c = choose(nodes, seg, N, nw);
+  {
+    std::lock_guard<std::mutex> lk(g_plan_mu);
+    if (plan_cache().count(c.key)) return true;
+  }
+  for (const Part& p : split(nodes, seg, c.sched.cut_adds, c.sched.layout >= 1 ? 1 : 32)) {
+    if ((p.order.empty() && p.pops.empty()) || p.lookback_add) continue;
+    if (p.inputs.size() > kMaxInputs) return false;
+    {
+      std::lock_guard<std::mutex> lk(g_part_mu);
+      if (part_cache().count(part_key(nodes, p, (N % 64) != 0, c.sched))) continue;
+    }
+    Schedule sc = c.sched;
+    PartKernel pk;
+    if (!is_compiled(part_source(nodes, p, N, sc, pk))) return false;
+  }
+  return true;
+}
+
+int64_t FusedBackend::prepare(const std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
+                              double* compile_ms) {
+  using clk = std::chrono::steady_clock;
+  auto ms_since = [](clk::time_point t) { return std::chrono::duration<double, std::milli>(clk::now() - t).count(); };
+  auto tp = clk::now();
+  Choice choice = choose(nodes, seg, N, nw);
+  const std::string& skey = choice.key;
+  const Schedule& sc = choice.sched;
   std::shared_ptr<const SegPlan> plan;
   {
     std::lock_guard<std::mutex> lk(g_plan_mu);
@@ -2043,7 +2046,7 @@ int64_t FusedBackend::prepare(const std::vector<Node>& nodes, const Segment& seg
   resolve();
   impl_->plan = plan;
   impl_->plan_sched = sc;
-  impl_->plan_spec_key = std::move(spec_key);
+  impl_->plan_spec_key = std::move(choice.spec_key);
   t_prelaunch_ms += ms_since(tp);
   return static_cast<int64_t>(plan->parts.size());
 }

@@ -54,7 +54,7 @@ class FusedBackend {
   void set_schedule(const Schedule& s);
   // True when every kernel `run` would launch for this segment is already
   // compiled (in this process or in the on-disk kernel cache).
-  bool all_compiled(const std::vector<Node>& nodes, const Segment& seg, int64_t N);
+  bool all_compiled(const std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw);
 
   int64_t fallbacks = 0;   // parts re-run with the plain kernels (speculation unproven)
   int64_t launches = 0;    // fused kernels launched
@@ -65,6 +65,12 @@ class FusedBackend {
   struct Impl;
 
  private:
+  struct Choice {
+    Schedule sched;
+    std::string key;        // of the segment's plan
+    std::string spec_key;   // non-empty: its additions speculate
+  };
+  Choice choose(const std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw) const;
   std::unique_ptr<Impl> impl_;
 };
 
