@@ -19,9 +19,10 @@
 //    above the first clean bit where its operands are equal, which decides the
 //    carry; shifts move the dirt by their distance).  If the dirt has died out
 //    before the range starts the state is exact; otherwise the warm-up is
-//    doubled (up to 8 times).  If it still cannot be proven exact the kernel
-//    raises a flag and the host re-runs the segment with the plain per-op
-//    kernels, which are exact by construction.
+//    doubled, up to the reach (kReach).  If it still cannot be proven exact the
+//    kernel raises a flag and the host re-runs the segment: in the warp form,
+//    which reaches further, if it ran in a thread form that no caller asked
+//    for; else with the plain per-op kernels, exact by construction.
 //  * Right shifts of temporaries and left shifts of temporaries by 2048 bits
 //    or more need words the warp has not computed yet / no longer holds; the
 //    segment is cut there: the operand is materialized by an earlier kernel.
@@ -158,6 +159,14 @@ struct Part {
 // really happens is tracked on the device.
 constexpr int64_t kAddSettle = 4;
 
+// How far back a warm-up is doubled before its range counts as unproven: this
+// many times 64 words in the warp form, 4 in the thread forms, more where
+// shifts alone take longer (Gen::reach).  Not a multiple of the first warm-up,
+// which is as short as the DAG's usual dirt: a carry that propagates through
+// 12,000 words is proven by going back that far, and the whole segment is run
+// again one operation at a time if it is not.
+constexpr int64_t kReach = 256;
+
 // One kernel of the warp form.  Dirt is tracked in bits, not words: a chain of 40 one-bit shifts and 20
 // additions dirties about 120 bits, which 4 warm-up words settle; counted as
 // one word per operation it took 64 words and four doublings (a 200-op DAG of
@@ -202,6 +211,7 @@ struct Gen {
   std::vector<uint8_t> dyn;        // node dirt must be tracked during warm-up
   std::map<int, int64_t> sdh;      // static dirt (bits) for nodes without add ancestors
   int64_t warm = 32;               // warm-up words
+  int64_t reach = 0;               // words that the doubled warm-ups go back at least
   // Global loads of one step ("load slots"): expression templates over @W@
   // (this lane's word) and @B@ (the step's first word), de-duplicated.  The
   // owned-range loop issues them one step ahead of the arithmetic.
@@ -286,8 +296,9 @@ struct Gen {
       for (size_t i = 0; i < part.outputs.size(); ++i) outs.push_back({part.outputs[i], static_cast<int>(i)});
     for (int n : part.order) in_part.insert(n);
     dyn.assign(nodes.size(), 0);
-    int64_t max_dirt = 0;
+    int64_t max_dirt = 0, max_words = 0;
     std::map<int, int64_t> likely;   // dirt (bits), additions taken to settle in kAddSettle
+    std::map<int, int64_t> words;    // in words, one at least per shift, of what no addition is part of
     for (int n : part.order) {
       const Node& x = nodes[n];
       auto d = [&](const std::map<int, int64_t>& m, int o) -> int64_t {
@@ -311,11 +322,16 @@ struct Gen {
         shift = x.k;
       }
       dyn[n] = dy;
-      if (!dy) sdh[n] = std::max(d(sdh, x.a), d(sdh, x.b)) + shift;
+      if (!dy) {
+        sdh[n] = std::max(d(sdh, x.a), d(sdh, x.b)) + shift;
+        words[n] = std::max(d(words, x.a), d(words, x.b)) + (shift + 63) / 64;
+        max_words = std::max(max_words, words[n]);
+      }
       likely[n] = std::max(d(likely, x.a), d(likely, x.b)) + shift + (x.op == NOp::Add ? kAddSettle : 0);
       max_dirt = std::max(max_dirt, likely[n]);
     }
     warm = std::min<int64_t>(8192, ((max_dirt + 63) / 64 + 1 + 31) / 32 * 32);
+    reach = kReach * std::min<int64_t>(8192, (max_words + 64 + 31) / 32 * 32);
     int nb = 0;
     for (int n : part.order)
       if (nodes[n].op == NOp::Add) cbit[n] = nb++;
@@ -689,7 +705,7 @@ struct Gen {
     if (need_warm) {
       s << "  const long long H = " << warm << ";\n"
         << "  long long p0 = s - H;\n  if (p0 < 0) p0 = 0;\n"
-        << "  for (int attempt = 0; p0 < s; ++attempt) {\n";
+        << "  while (p0 < s) {\n";
       for (int i = 0; i < n_pack; ++i) s << "    pk" << i << " = 0;\n";
       for (int n : shl_src)
         if (!small_shl.count(n)) s << "    pv" << n << " = 0;\n";
@@ -711,7 +727,7 @@ struct Gen {
           s << "    ok = ok && " << sdh.at(n) << " <= need - " << shl_k.at(n) << ";\n";
       }
       s << "    if (ok || p0 == 0) break;\n"
-        << "    if (attempt >= 8) { if (lane == 0) atomicOr(A.fail, 1u); break; }\n"
+        << "    if (s - p0 >= " << reach << "ll) { if (lane == 0) atomicOr(A.fail, 1u); break; }\n"
         << "    p0 = s - 2 * (s - p0);\n    if (p0 < 0) p0 = 0;\n"
         << "  }\n";
     }
@@ -775,8 +791,8 @@ struct Gen {
 // (and any chunk whose shifted loads would leave [0, nw)) take a scalar path
 // with bounds, tail fill and last-word masking.  The state at the start of a
 // thread's range comes from speculation as in the warp form: H warm-up words
-// from an all-zero state, per-node dirt tracking in bits, doubled up to 8
-// times, then the fail flag and the exact per-op fallback.
+// from an all-zero state, per-node dirt tracking in bits, doubled up to the
+// reach, then the fail flag.
 struct GenSeq {
   const std::vector<Node>& nodes;
   const Part& part;
@@ -792,6 +808,7 @@ struct GenSeq {
   std::map<int, int64_t> sdh;        // static dirt (bits) of nodes without add ancestors
   std::map<int, int64_t> prev_k;     // max shift (bits) of the nodes in prev_src
   int64_t warm = 4;                  // warm-up words (multiple of 4)
+  int64_t reach = 0;                 // as in the warp form
   std::vector<int> emit_order;
   // shifted input reads by a word offset: (node, word offset) -> slot; the
   // offset is -ws for a left shift and +ws for a right shift (|ws| >= 1 for
@@ -837,7 +854,7 @@ struct GenSeq {
     // Dirt in bits: a value exact from bit B shifted left by k < 64 is exact
     // from bit B + k.
     std::map<int, int64_t> likely;   // as in the warp form
-    int64_t max_dirt = 0;
+    int64_t max_dirt = 0, max_static = 0;
     for (int n : part.order) {
       const Node& x = nodes[n];
       auto d = [&](const std::map<int, int64_t>& m, int o) -> int64_t {
@@ -875,11 +892,15 @@ struct GenSeq {
       }
       if (shift) prev_k[x.a] = std::max(prev_k[x.a], shift);
       dyn[n] = dy;
-      if (!dy) sdh[n] = std::max(d(sdh, x.a), d(sdh, x.b)) + shift;
+      if (!dy) {
+        sdh[n] = std::max(d(sdh, x.a), d(sdh, x.b)) + shift;
+        max_static = std::max(max_static, sdh[n]);
+      }
       likely[n] = std::max(d(likely, x.a), d(likely, x.b)) + shift + (x.op == NOp::Add ? kAddSettle : 0);
       max_dirt = std::max(max_dirt, likely[n]);
     }
     warm = ((max_dirt + 63) / 64 + 1 + 3) / 4 * 4;
+    reach = kReach * std::max<int64_t>(4, ((max_static + 63) / 64 + 2 + 3) / 4 * 4);
     int k = 0;
     for (auto& kv : off_slot) {
       kv.second = k++;
@@ -1158,7 +1179,7 @@ struct GenSeq {
       << "      const int q = ch % " << stages << ";\n"
       << "      if (issued < nch) { issue(issued, issued % " << stages << "); ++issued; }\n"
       // bounded wait; a stage that never lands sets the fail flag (the host
-      // then re-runs the part with the exact per-op kernels)
+      // then re-runs the part in another form)
       << "      {\n        const unsigned mb = smem_u32(&bar[warp][q]);\n        unsigned done = 0;\n"
       << "        for (int it = 0; it < (1 << 22) && !done; ++it)\n"
       << "          asm volatile(\"{ .reg .pred p; mbarrier.try_wait.parity.shared.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }\" "
@@ -1343,7 +1364,7 @@ struct GenSeq {
     // ---- warm-up
     if (!adds.empty() || !prev_src.empty()) {
       s << "  long long p0 = s - " << warm << "ll;\n  if (p0 < 0) p0 = 0;\n"
-        << "  for (int attempt = 0; p0 < s; ++attempt) {\n";
+        << "  while (p0 < s) {\n";
       for (int n : adds) s << "    cy" << n << " = 0;\n";
       for (int n : prev_src) s << "    pv" << n << " = 0;\n";
       for (int n : adds)
@@ -1362,7 +1383,7 @@ struct GenSeq {
           s << "    ok = ok && " << sdh.at(n) << " <= need - " << prev_k.at(n) << ";\n";
       }
       s << "    if (ok || p0 == 0) break;\n"
-        << "    if (attempt >= 8) { atomicOr(A.fail, 1u); break; }\n"
+        << "    if (s - p0 >= " << reach << "ll) { atomicOr(A.fail, 1u); break; }\n"
         << "    p0 = s - 2 * (s - p0);\n    if (p0 < 0) p0 = 0;\n"
         << "  }\n";
     }
@@ -1854,6 +1875,8 @@ struct PendingSegment {
   int64_t N = 0, nw = 0;
   unsigned long long* d_slots = nullptr;
   std::string spec_key;   // non-empty: the segment ran with speculative carries (scheme 0)
+  Segment seg;            // kept if the warp form may take over (a thread form that no caller chose)
+  bool warp_next = false;
 };
 
 // Segments (graph and schedule keys) whose speculative carry state could not
@@ -1867,6 +1890,25 @@ std::unordered_set<std::string>& spec_failed() {
   return s;
 }
 
+// Segments (keyed as above) whose speculation failed in a thread form that the
+// executor had chosen: from then on they take the warp form, which proves
+// carries that propagate 16 times as far (a warp takes 32 words of a warm-up
+// at a time, so that it can go back 16,384 words and more).
+std::unordered_set<std::string>& threads_failed() {
+  static std::unordered_set<std::string> s;
+  return s;
+}
+
+bool failed_before(const std::unordered_set<std::string>& set, const std::string& key) {
+  std::lock_guard<std::mutex> lk(g_spec_mu);
+  return set.count(key) != 0;
+}
+void note_failed(std::unordered_set<std::string>& set, const std::string& key) {
+  std::lock_guard<std::mutex> lk(g_spec_mu);
+  if (set.size() >= kMaxPlans) set.clear();
+  set.insert(key);
+}
+
 struct FusedBackend::Impl {
   Device& dev;
   ExecOptions opt;
@@ -1875,8 +1917,7 @@ struct FusedBackend::Impl {
   std::unique_ptr<PendingSegment> pending;
   // from prepare() to run()
   std::shared_ptr<const SegPlan> plan;
-  Schedule plan_sched;
-  std::string plan_spec_key;
+  Choice choice;
   Impl(Device& d, const ExecOptions& o) : dev(d), opt(o) {}
 };
 
@@ -1980,13 +2021,15 @@ FusedBackend::Choice FusedBackend::choose(const std::vector<Node>& nodes, const 
     return graph_key(nodes, seg.order, seg.inputs, seg.outputs, seg.pops, (N % 64) != 0, c.sched);
   };
   c.key = key();
-  if (c.sched.cut_adds == 0) {
-    bool failed_before;
-    {
-      std::lock_guard<std::mutex> lk(g_spec_mu);
-      failed_before = spec_failed().count(c.key) != 0;
+  if (!impl_->scheduled && c.sched.layout >= 1) {
+    c.warp_next = !failed_before(threads_failed(), c.key);
+    if (!c.warp_next) {
+      c.sched = Schedule{};
+      c.key = key();
     }
-    if (failed_before) {
+  }
+  if (c.sched.cut_adds == 0) {
+    if (failed_before(spec_failed(), c.key)) {
       c.sched.cut_adds = 2;
       c.key = key();
     } else {
@@ -2016,56 +2059,52 @@ bool FusedBackend::all_compiled(const std::vector<Node>& nodes, const Segment& s
   return true;
 }
 
+namespace {
+
+std::shared_ptr<const SegPlan> plan_for(const std::vector<Node>& nodes, const Segment& seg, int64_t N,
+                                        const Schedule& sc, const std::string& key, double* compile_ms) {
+  {
+    std::lock_guard<std::mutex> lk(g_plan_mu);
+    auto it = plan_cache().find(key);
+    if (it != plan_cache().end()) return it->second;
+  }
+  auto plan = std::make_shared<SegPlan>();
+  for (Part& p : split(nodes, seg, sc.cut_adds, sc.layout >= 1 ? 1 : 32)) {
+    if (p.order.empty() && p.pops.empty()) continue;
+    if (p.inputs.size() > kMaxInputs) throw RuntimeError("fused: too many inputs in one segment");
+    plan->kernels.push_back(p.lookback_add ? PartKernel{} : part_kernel(nodes, p, N, sc, compile_ms));
+    plan->parts.push_back(std::move(p));
+  }
+  std::lock_guard<std::mutex> lk(g_plan_mu);
+  if (plan_cache().size() >= kMaxPlans) plan_cache().clear();
+  plan_cache()[key] = plan;
+  return plan;
+}
+
+}  // namespace
+
 int64_t FusedBackend::prepare(const std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
                               double* compile_ms) {
   using clk = std::chrono::steady_clock;
   auto ms_since = [](clk::time_point t) { return std::chrono::duration<double, std::milli>(clk::now() - t).count(); };
   auto tp = clk::now();
-  Choice choice = choose(nodes, seg, N, nw);
-  const std::string& skey = choice.key;
-  const Schedule& sc = choice.sched;
-  std::shared_ptr<const SegPlan> plan;
-  {
-    std::lock_guard<std::mutex> lk(g_plan_mu);
-    auto it = plan_cache().find(skey);
-    if (it != plan_cache().end()) plan = it->second;
-  }
-  if (!plan) {
-    auto np = std::make_shared<SegPlan>();
-    for (Part& p : split(nodes, seg, sc.cut_adds, sc.layout >= 1 ? 1 : 32)) {
-      if (p.order.empty() && p.pops.empty()) continue;
-      if (p.inputs.size() > kMaxInputs) throw RuntimeError("fused: too many inputs in one segment");
-      np->kernels.push_back(p.lookback_add ? PartKernel{} : part_kernel(nodes, p, N, sc, compile_ms));
-      np->parts.push_back(std::move(p));
-    }
-    std::lock_guard<std::mutex> lk(g_plan_mu);
-    if (plan_cache().size() >= kMaxPlans) plan_cache().clear();
-    plan_cache()[skey] = np;
-    plan = np;
-  }
+  impl_->choice = choose(nodes, seg, N, nw);
+  impl_->plan = plan_for(nodes, seg, N, impl_->choice.sched, impl_->choice.key, compile_ms);
   resolve();
-  impl_->plan = plan;
-  impl_->plan_sched = sc;
-  impl_->plan_spec_key = std::move(choice.spec_key);
   t_prelaunch_ms += ms_since(tp);
-  return static_cast<int64_t>(plan->parts.size());
+  return static_cast<int64_t>(impl_->plan->parts.size());
 }
 
-bool FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
-                       unsigned long long* d_slots, unsigned int* d_flags, const SlotPublish& pub) {
-  (void)seg;
+namespace {
+
+// Launches a plan's parts; `d_flags`: a zeroed word for each.  Returns true if
+// the last kernel does what `pub` says.
+bool launch_plan(Device& dev, std::vector<Node>& nodes, const SegPlan& plan, const Schedule& sc, int64_t N, int64_t nw,
+                 unsigned long long* d_slots, unsigned int* d_flags, const SlotPublish& pub) {
   bool published = false;
-  Device& dev = impl_->dev;
-  const std::shared_ptr<const SegPlan> plan = std::move(impl_->plan);
-  const Schedule& sc = impl_->plan_sched;
-  std::string spec_key = std::move(impl_->plan_spec_key);
-  impl_->d_fail = d_flags;
-  using clk = std::chrono::steady_clock;
-  auto ms_since = [](clk::time_point t) { return std::chrono::duration<double, std::milli>(clk::now() - t).count(); };
-  auto tp = clk::now();
-  for (size_t pi = 0; pi < plan->parts.size(); ++pi) {
-    const Part& p = plan->parts[pi];
-    const PartKernel& pk = plan->kernels[pi];
+  for (size_t pi = 0; pi < plan.parts.size(); ++pi) {
+    const Part& p = plan.parts[pi];
+    const PartKernel& pk = plan.kernels[pi];
     const Compiled& c = pk.c;
     // outputs
     for (int n : p.outputs)
@@ -2143,7 +2182,7 @@ bool FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
       uint64_t* tail = reinterpret_cast<uint64_t*>(targs.data() + maps_bytes);
       for (int i = 0; i < ni + no; ++i) tail[i] = args[i];
       tail[ni + no + 0] = reinterpret_cast<uint64_t>(d_slots);
-      tail[ni + no + 1] = reinterpret_cast<uint64_t>(impl_->d_fail + pi);
+      tail[ni + no + 1] = reinterpret_cast<uint64_t>(d_flags + pi);
       tail[ni + no + 2] = static_cast<uint64_t>(nw);
       tail[ni + no + 3] = static_cast<uint64_t>(range);
       tail[ni + no + 4] = mask_for_bits(N);
@@ -2191,12 +2230,12 @@ bool FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
       if (sc.ctas_per_sm > 0) blocks = std::min<int>(blocks, dev.sm_count() * per_sm);
     }
     args[ni + no + 0] = reinterpret_cast<uint64_t>(d_slots);
-    args[ni + no + 1] = reinterpret_cast<uint64_t>(impl_->d_fail + pi);
+    args[ni + no + 1] = reinterpret_cast<uint64_t>(d_flags + pi);
     args[ni + no + 2] = static_cast<uint64_t>(nw);
     args[ni + no + 3] = static_cast<uint64_t>(range);
     args[ni + no + 4] = mask_for_bits(N);
     const int resident = pk.roww > 0 ? pk.tma_blocks_per_sm : c.blocks_per_sm;
-    if (pi + 1 == plan->parts.size() && pub.n > 0 && blocks <= static_cast<int64_t>(dev.sm_count()) * resident) {
+    if (pi + 1 == plan.parts.size() && pub.n > 0 && blocks <= static_cast<int64_t>(dev.sm_count()) * resident) {
       uint64_t* f = pk.roww > 0 ? reinterpret_cast<uint64_t*>(targs.data() + publish_at) : args.data() + ni + no + 6;
       f[0] = reinterpret_cast<uint64_t>(pub.host);
       f[1] = reinterpret_cast<uint64_t>(pub.from);
@@ -2211,10 +2250,25 @@ bool FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
                             reinterpret_cast<CUstream>(dev.stream()), kparams, nullptr));
     }
     ++dev.n_launches;
-    ++launches;
-    t_prelaunch_ms += ms_since(tp);
-    tp = clk::now();
   }
+  return published;
+}
+
+int64_t generated_parts(const SegPlan& plan) {
+  return std::count_if(plan.parts.begin(), plan.parts.end(), [](const Part& p) { return !p.lookback_add; });
+}
+
+}  // namespace
+
+bool FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
+                       unsigned long long* d_slots, unsigned int* d_flags, const SlotPublish& pub) {
+  using clk = std::chrono::steady_clock;
+  const auto t0 = clk::now();
+  const std::shared_ptr<const SegPlan> plan = std::move(impl_->plan);
+  Choice& choice = impl_->choice;
+  impl_->d_fail = d_flags;
+  const bool published = launch_plan(impl_->dev, nodes, *plan, choice.sched, N, nw, d_slots, d_flags, pub);
+  launches += generated_parts(*plan);
   // the segment stays pending until resolve()
   auto pend = std::make_unique<PendingSegment>();
   pend->plan = plan;
@@ -2222,8 +2276,11 @@ bool FusedBackend::run(std::vector<Node>& nodes, const Segment& seg, int64_t N, 
   pend->N = N;
   pend->nw = nw;
   pend->d_slots = d_slots;
-  pend->spec_key = std::move(spec_key);
+  pend->spec_key = std::move(choice.spec_key);
+  pend->warp_next = choice.warp_next;
+  if (pend->warp_next) pend->seg = seg;
   impl_->pending = std::move(pend);
+  t_prelaunch_ms += std::chrono::duration<double, std::milli>(clk::now() - t0).count();
   return published;
 }
 
@@ -2296,26 +2353,49 @@ void FusedBackend::resolve() {
 bool FusedBackend::resolve_with(const uint32_t* flags) {
   if (!impl_->pending) return false;
   std::unique_ptr<PendingSegment> pend = std::move(impl_->pending);
-  const std::vector<Part>& parts = *pend->parts;
-  size_t first = parts.size();
-  for (size_t i = 0; i < parts.size(); ++i)
-    if (flags[i]) {
-      first = i;
-      break;
+  Device& dev = impl_->dev;
+  auto unproven = [](const uint32_t* f, size_t k) {
+    return static_cast<size_t>(std::find_if(f, f + k, [](uint32_t x) { return x != 0; }) - f);
+  };
+  size_t n = pend->parts->size(), first = unproven(flags, n);
+  if (first == n) return false;
+  std::vector<uint32_t> warp_flags;
+  std::shared_ptr<const SegPlan> warp_plan;
+  if (pend->warp_next) {
+    // the same segment in the warp form, which proves more
+    note_failed(threads_failed(), pend->spec_key);
+    const Segment& seg = pend->seg;
+    const Schedule sc{};
+    const std::string key =
+        graph_key(pend->nodes, seg.order, seg.inputs, seg.outputs, seg.pops, (pend->N % 64) != 0, sc);
+    if (!failed_before(spec_failed(), key)) {
+      warp_plan = plan_for(pend->nodes, seg, pend->N, sc, key, nullptr);
+      n = warp_plan->parts.size();
+      warp_flags.resize(n);
+      for (auto& pp : seg.pops) BSZ_CUDA(cudaMemsetAsync(pend->d_slots + pp.second, 0, 8, dev.stream()));
+      const BufRef mem = dev.alloc_stream(static_cast<int64_t>(n + 1) / 2);
+      auto* d_flags = reinterpret_cast<unsigned int*>(mem->p);
+      BSZ_CUDA(cudaMemsetAsync(d_flags, 0, 4 * n, dev.stream()));
+      launch_plan(dev, pend->nodes, *warp_plan, sc, pend->N, pend->nw, pend->d_slots, d_flags, SlotPublish{});
+      launches += generated_parts(*warp_plan);
+      BSZ_CUDA(cudaMemcpyAsync(warp_flags.data(), d_flags, 4 * n, cudaMemcpyDeviceToHost, dev.stream()));
+      BSZ_CUDA(cudaStreamSynchronize(dev.stream()));
+      flags = warp_flags.data();
+      first = unproven(flags, n);
+      if (first == n) return true;
+      pend->spec_key = key;
+      pend->parts = &warp_plan->parts;
     }
+  }
   // Speculation could not be proven exact in part `first`: redo it, and
   // every later part (which may have read its outputs), with the plain
   // per-op kernels (exact by construction).
-  for (size_t i = first; i < parts.size(); ++i) {
-    rerun_part_exact(impl_->dev, parts[i], pend->nodes, pend->N, pend->nw, pend->d_slots);
+  for (size_t i = first; i < n; ++i) {
+    rerun_part_exact(dev, (*pend->parts)[i], pend->nodes, pend->N, pend->nw, pend->d_slots);
     if (flags[i]) ++fallbacks;
   }
-  if (first < parts.size() && !pend->spec_key.empty()) {
-    std::lock_guard<std::mutex> lk(g_spec_mu);
-    if (spec_failed().size() >= kMaxPlans) spec_failed().clear();
-    spec_failed().insert(pend->spec_key);
-  }
-  return first < parts.size();
+  if (!pend->spec_key.empty()) note_failed(spec_failed(), pend->spec_key);
+  return true;
 }
 
 // ================================================================ batches ==

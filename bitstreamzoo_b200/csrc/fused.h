@@ -37,9 +37,11 @@ class FusedBackend {
   int64_t prepare(const std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw, double* compile_ms);
   bool run(std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw,
            unsigned long long* d_slots, unsigned int* d_flags, const SlotPublish& pub);
-  // Waits for the pending segment, reads its parts' flags and re-runs every
-  // part from the first unproven one on with the exact per-op kernels (a
-  // later part may have read the unproven part's outputs).  Must be called
+  // Waits for the pending segment, reads its parts' flags and re-runs what is
+  // unproven: the segment in the warp form if it ran in a thread form that the
+  // executor had picked; else, or if that fails too, every part from the first
+  // unproven one on with the exact per-op kernels (a later part may have read
+  // the unproven part's outputs).  Must be called
   // before anything reads the segment's outputs or popcounts or launches
   // work that depends on them; a no-op when nothing is pending.
   void resolve();
@@ -69,6 +71,7 @@ class FusedBackend {
     Schedule sched;
     std::string key;        // of the segment's plan
     std::string spec_key;   // non-empty: its additions speculate
+    bool warp_next = false; // if it fails, the warp form is tried before the per-op kernels
   };
   Choice choose(const std::vector<Node>& nodes, const Segment& seg, int64_t N, int64_t nw) const;
   std::unique_ptr<Impl> impl_;
