@@ -567,6 +567,7 @@ bool Executor::nonzero(int node, const Stmt* at) {
   unsigned int h = 0;
   BSZ_CUDA(cudaMemcpyAsync(&h, d_flag_, 4, cudaMemcpyDeviceToHost, dev_.stream()));
   dev_.sync();
+  hold_.clear();
   ++n_syncs;
   check_error();
   return h != 0;
@@ -1299,6 +1300,7 @@ void Executor::settle() {
     BSZ_CUDA(cudaMemcpyAsync(block.get(), d_slots_ + (first - slot_base_), bytes, cudaMemcpyDeviceToHost,
                              dev_.stream()));
     BSZ_CUDA(cudaStreamSynchronize(dev_.stream()));
+    hold_.clear();
     std::memcpy(slot_val_.data() + first, block.get(), bytes);
     ++n_syncs;
   };
@@ -1306,6 +1308,7 @@ void Executor::settle() {
   if (first < n_slots_) {
     if (published_ && published_from_ == first && published_count_ == n_slots_ - first) {
       BSZ_CUDA(cudaStreamSynchronize(dev_.stream()));
+      hold_.clear();
       std::memcpy(slot_val_.data() + first, published_.get(), static_cast<size_t>(published_count_) * 8);
       ++n_syncs;
     } else {

@@ -230,8 +230,8 @@ class Executor {
   int64_t pub_cap_ = 0;
   int64_t zeroed_ = 0;               // slots below this are zero or in use
   // Page-locked blocks that enqueued kernels read or write: kept until the
-  // run has finished (the device's buffers are reused in stream order, host
-  // memory is not).
+  // stream has been waited for (the device's buffers are reused in stream
+  // order, host memory is not).
   std::vector<std::shared_ptr<void>> hold_;
   std::shared_ptr<void> err_word_;   // this run's device error word
   uint32_t* error_word() const { return static_cast<uint32_t*>(err_word_.get()); }
