@@ -126,9 +126,9 @@ k_gemm(const float* __restrict__ A, const float* __restrict__ B, float* __restri
   float* As = s_mem;
   float* Bs = s_mem + kChunk * kPad;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int m0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
+  const int m0 = blockIdx.x * kTile, n0 = blockIdx.y * kTile;
   const int tm = (lane >> 2) * 4, tn = (lane & 3) * 8;   // this lane's 4 x 8 outputs
-  const bool sums = colsum != nullptr && blockIdx.y == 0;
+  const bool sums = colsum != nullptr && blockIdx.x == 0;
   float acc[4][8] = {};
   float cs = 0.f;
   for (int k0 = 0; k0 < K; k0 += kChunk) {
@@ -226,7 +226,8 @@ void check(cudaError_t e, const char* what) {
 template <int TA, int TB>
 void gemm(cudaStream_t s, const float* A, const float* B, float* C, const float* bias, const float* mask,
           float* colsum, int M, int N, int K, int relu) {
-  dim3 grid((N + kTile - 1) / kTile, (M + kTile - 1) / kTile);
+  // rows along x: a grid has 65,535 blocks along y, two million rows
+  dim3 grid((M + kTile - 1) / kTile, (N + kTile - 1) / kTile);
   launch_after(s, grid, kGemmWarps * 32, kGemmSmem, k_gemm<TA, TB>, A, B, C, bias, mask, colsum, M, N, K, relu);
   check(cudaGetLastError(), "mlp gemm launch");
 }
