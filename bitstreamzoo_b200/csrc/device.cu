@@ -47,33 +47,39 @@ Device::~Device() {
     for (cudaEvent_t e : pool) cudaEventDestroy(e);
   if (d_scratch_) cudaFree(d_scratch_);
   arena_.reset();
-  for (auto& kv : *pinned_free_) cudaFreeHost(kv.second);
-  pinned_free_->clear();
+  for (auto& kv : pinned_->free) cudaFreeHost(kv.second);
+  pinned_->free.clear();
   copies_.reset();
   if (stream_) cudaStreamDestroy(stream_);
 }
 
-constexpr size_t kMaxPinnedFree = 512;   // cached blocks; a run takes up to a few dozen
+// Cached blocks: a run takes up to a few dozen, of some hundred KiB at most.
+constexpr size_t kMaxPinnedFree = 512, kMaxPinnedBytes = size_t(64) << 20;
 
 std::shared_ptr<void> Device::pinned_block(size_t bytes) {
   bytes = std::max<size_t>(4096, (bytes + 4095) / 4096 * 4096);
   void* p = nullptr;
   size_t have = bytes;
-  auto it = pinned_free_->lower_bound(bytes);
-  if (it != pinned_free_->end() && it->first <= 4 * bytes) {
+  auto it = pinned_->free.lower_bound(bytes);
+  if (it != pinned_->free.end() && it->first <= 4 * bytes) {
     have = it->first;
     p = it->second;
-    pinned_free_->erase(it);
+    pinned_->free.erase(it);
+    pinned_->bytes -= have;
   } else {
     BSZ_CUDA(cudaHostAlloc(&p, bytes, cudaHostAllocDefault));
   }
   // the cache outlives the Device only through blocks still referenced:
   // those are freed directly when the Device is gone
-  std::weak_ptr<std::multimap<size_t, void*>> pool = pinned_free_;
-  return std::shared_ptr<void>(p, [pool, have](void* q) {
-    auto m = pool.lock();
-    if (m && m->size() < kMaxPinnedFree) m->emplace(have, q);
-    else cudaFreeHost(q);
+  std::weak_ptr<PinnedCache> cache = pinned_;
+  return std::shared_ptr<void>(p, [cache, have](void* q) {
+    auto c = cache.lock();
+    if (c && c->free.size() < kMaxPinnedFree && c->bytes + have <= kMaxPinnedBytes) {
+      c->free.emplace(have, q);
+      c->bytes += have;
+    } else {
+      cudaFreeHost(q);
+    }
   });
 }
 

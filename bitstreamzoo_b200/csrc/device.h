@@ -150,7 +150,11 @@ class Device {
   std::vector<cudaEvent_t> events_[2];
   void* d_scratch_ = nullptr;
   size_t scratch_cap_ = 0;
-  std::shared_ptr<std::multimap<size_t, void*>> pinned_free_ = std::make_shared<std::multimap<size_t, void*>>();
+  struct PinnedCache {
+    std::multimap<size_t, void*> free;   // by size
+    size_t bytes = 0;
+  };
+  std::shared_ptr<PinnedCache> pinned_ = std::make_shared<PinnedCache>();
   std::shared_ptr<void> arena_;   // the block that host_slice cuts from
   size_t arena_used_ = 0;
   std::unique_ptr<class CopyPool> copies_;   // made by the first large copy

@@ -301,23 +301,47 @@ void Mlp::ensure(int n) {
   }
 }
 
-// The block comes from the device's pool and goes back when the call, which
-// waits for its results, returns: one of the model's own took its first call
-// 2.5 ms to allocate.
-std::shared_ptr<float> Mlp::upload(const float* x, const float* y, int n) {
+// Rows, targets and results of a call pass through a page-locked block while
+// they are small: a copy from or into the caller's pageable memory by the
+// driver takes several times as long.  The block comes from the device's pool
+// and goes back when the call, which waits for its results, returns: one of the
+// model's own took its first call 2.5 ms to allocate.  Past kMaxBlock the
+// device's ring of copy buffers does it, whose size does not follow the rows'.
+constexpr size_t kMaxBlock = size_t(4) << 20;
+
+Mlp::Block Mlp::upload(const float* x, const float* y, int n) {
   ensure(n);
   const size_t results = 1 + std::max<size_t>(static_cast<size_t>(n_params_), static_cast<size_t>(n));
-  const std::shared_ptr<void> raw = dev_.pinned_block(4 * (results + static_cast<size_t>(n) * (dims_[0] + 1)));
-  std::shared_ptr<float> block(raw, static_cast<float*>(raw.get()));
-  float* h = block.get() + results;
-  const size_t nx = static_cast<size_t>(n) * dims_[0];
+  const size_t nx = static_cast<size_t>(n) * dims_[0], ny = y ? static_cast<size_t>(n) : 0;
+  const bool small = 4 * (results + nx + ny) <= kMaxBlock;
+  Block b;
+  b.mem = dev_.pinned_block(small ? 4 * (results + nx + ny) : 4);
+  b.loss = static_cast<float*>(b.mem.get());
+  if (!small) {
+    dev_.h2d(x_, x, nx * 4);
+    dev_.h2d(y_, y, ny * 4);
+    return b;
+  }
+  b.out = b.loss + 1;
+  float* h = b.loss + results;
   std::memcpy(h, x, nx * 4);
   check(cudaMemcpyAsync(x_, h, nx * 4, cudaMemcpyHostToDevice, stream_), "mlp upload");
   if (y) {
-    std::memcpy(h + nx, y, static_cast<size_t>(n) * 4);
-    check(cudaMemcpyAsync(y_, h + nx, static_cast<size_t>(n) * 4, cudaMemcpyHostToDevice, stream_), "mlp upload");
+    std::memcpy(h + nx, y, ny * 4);
+    check(cudaMemcpyAsync(y_, h + nx, ny * 4, cudaMemcpyHostToDevice, stream_), "mlp upload");
   }
-  return block;
+  return b;
+}
+
+void Mlp::download(const Block& b, float* dst, const float* src, size_t n) {
+  if (!b.out) {
+    dev_.d2h(dst, src, n * 4);
+    check(cudaStreamSynchronize(stream_), "mlp download");
+    return;
+  }
+  check(cudaMemcpyAsync(b.out, src, n * 4, cudaMemcpyDeviceToHost, stream_), "mlp download");
+  check(cudaStreamSynchronize(stream_), "mlp download");
+  std::memcpy(dst, b.out, n * 4);
 }
 
 void Mlp::forward(int n) {
@@ -351,11 +375,11 @@ void Mlp::backward(int n, float* loss) {
 }
 
 float Mlp::train_step(const float* x, const float* y, int n, float lr) {
-  const std::shared_ptr<float> block = upload(x, y, n);
+  const Block block = upload(x, y, n);
   forward(n);
-  backward(n, block.get());
+  backward(n, block.loss);
   check(cudaStreamSynchronize(stream_), "mlp backward");
-  const float loss = *block;
+  const float loss = *block.loss;
   ++step_;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - std::pow(b1, static_cast<float>(step_));
@@ -367,27 +391,18 @@ float Mlp::train_step(const float* x, const float* y, int n, float lr) {
   return loss;
 }
 
-// Results come back through a page-locked block: a copy into the caller's
-// pageable memory by the driver takes several times as long.
 void Mlp::predict(const float* x, int n, float* out) {
-  const std::shared_ptr<float> block = upload(x, nullptr, n);
+  const Block block = upload(x, nullptr, n);
   forward(n);
-  float* h = block.get() + 1;
-  check(cudaMemcpyAsync(h, act_.back(), static_cast<size_t>(n) * 4, cudaMemcpyDeviceToHost, stream_), "mlp predict");
-  check(cudaStreamSynchronize(stream_), "mlp predict");
-  std::memcpy(out, h, static_cast<size_t>(n) * 4);
+  download(block, out, act_.back(), static_cast<size_t>(n));
 }
 
 float Mlp::gradients(const float* x, const float* y, int n, float* grad) {
-  const std::shared_ptr<float> block = upload(x, y, n);
+  const Block block = upload(x, y, n);
   forward(n);
-  backward(n, block.get());
-  float* h = block.get() + 1;
-  const size_t bytes = static_cast<size_t>(n_params_) * 4;
-  check(cudaMemcpyAsync(h, g_, bytes, cudaMemcpyDeviceToHost, stream_), "mlp grad");
-  check(cudaStreamSynchronize(stream_), "mlp grad");
-  std::memcpy(grad, h, bytes);
-  return *block;
+  backward(n, block.loss);
+  download(block, grad, g_, static_cast<size_t>(n_params_));
+  return *block.loss;
 }
 
 void Mlp::get_params(float* out) const {

@@ -48,9 +48,15 @@ class Mlp {
   Device& dev_;
   cudaStream_t stream_;
   void ensure(int n);
-  // A call's page-locked block: the loss, then predictions or gradients, then
-  // the inputs, which are on their way to the device.
-  std::shared_ptr<float> upload(const float* x, const float* y, int n);
+  // A call's page-locked block: the loss, then (where they are small) room for
+  // predictions or gradients and the inputs, on their way to the device.
+  struct Block {
+    std::shared_ptr<void> mem;
+    float* loss = nullptr;
+    float* out = nullptr;   // null: results are copied by the device's ring
+  };
+  Block upload(const float* x, const float* y, int n);
+  void download(const Block& b, float* dst, const float* src, size_t n);
   void forward(int n);
   void backward(int n, float* loss);   // leaves the loss on its way
 };

@@ -1,19 +1,25 @@
 """Page-locked host memory that runs and models keep."""
 
-import os
-
 import numpy as np
 import pytest
 
 import bitstreamzoo_b200 as bz
+from bitstreamzoo_b200 import tuner
 from bitstreamzoo_b200 import workloads as wl
 
 pytestmark = pytest.mark.gpu
 
 
-def _mapped_mib():
-    with open(f"/proc/{os.getpid()}/statm") as f:
-        return int(f.read().split()[0]) * os.sysconf("SC_PAGE_SIZE") / 2**20
+def _page_locked_mib():
+    """Page-locked host memory of this process: the driver maps it shared."""
+    with open("/proc/self/status") as f:
+        return next(int(line.split()[1]) for line in f if line.startswith("RssShmem:")) / 1024
+
+
+def _make_ring(ctx):
+    """The device's ring of copy buffers, made by the first large copy."""
+    a = wl.random_words(np.random.default_rng(2), 64 << 19)
+    ctx.run("input stream a\noutput stream o\no = ~a\n", 64 << 19, {"a": a}).stream("o")
 
 
 def test_a_long_walk_on_a_short_stream_keeps_no_list_per_segment(ctx):
@@ -37,7 +43,21 @@ def test_a_long_walk_on_a_short_stream_keeps_no_list_per_segment(ctx):
         return ctx.run(prog, nbits, ins | {"m": m}, mode=bz.MODE_VM)
 
     run(20)
-    before = _mapped_mib()
+    before = _page_locked_mib()
     r = run(trips)
     assert r.int("n") == trips and r.stats["n_vm_launches"] >= trips
-    assert _mapped_mib() - before < 20
+    assert _page_locked_mib() - before < 20
+
+
+def test_large_calls_of_the_cost_model_keep_no_page_locked_copy(ctx):
+    """48 MiB of rows in, 6 MiB of predictions out."""
+    n = 1_500_000
+    m = tuner.CostModel(ctx, 8, hidden=8, layers=1, seed=3)
+    x = np.random.default_rng(1).normal(0, 1, (n, 8)).astype(np.float32)
+    _make_ring(ctx)
+    few = m.raw_predict(x[:1000])
+    before = _page_locked_mib()
+    out = m.raw_predict(x)
+    del x
+    assert out.shape == (n,) and np.array_equal(out[:1000], few)
+    assert _page_locked_mib() - before < 20
