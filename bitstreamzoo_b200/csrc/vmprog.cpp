@@ -527,7 +527,7 @@ bool Executor::run_vm_program() {
     vm_buf_ = vm_mem_->p;
   }
   char* base = static_cast<char*>(vm_buf_);
-  hold_.push_back(dev_.host_slice(align(state_b) + ops_b));
+  hold_.push_back(dev_.host_slice(align(state_b) + (host_ops ? ops_b : 0)));
   char* host = static_cast<char*>(hold_.back().get());
   VmOp* list = reinterpret_cast<VmOp*>(host_ops ? host + align(state_b) : base);
   if (host_ops) std::memcpy(list, c.code.data(), ops_b);

@@ -61,3 +61,21 @@ def test_large_calls_of_the_cost_model_keep_no_page_locked_copy(ctx):
     del x
     assert out.shape == (n,) and np.array_equal(out[:1000], few)
     assert _page_locked_mib() - before < 20
+
+
+def test_a_long_program_takes_no_page_locked_memory_for_its_list(ctx):
+    """400,000 instructions with control flow, 6 MiB, run from device memory."""
+    body = "\n".join(f"x = x {'^' if i % 2 else '|'} {'ab'[i // 2 % 2]}" for i in range(400_000))
+    src = f"input stream a\ninput stream b\noutput stream x\nx = a\nif (a) {{\n{body}\n}}\n"
+    prog = ctx.compile(src)
+    ins = {"a": np.full(4, 5, dtype=np.uint64), "b": np.full(4, 9, dtype=np.uint64)}
+    _make_ring(ctx)
+    before = _page_locked_mib()
+    r = ctx.run(prog, 256, ins, mode=bz.MODE_VM)
+    assert r.stats["n_vm_launches"] == 1
+    want = 5
+    for i in range(400_000):
+        v = (5, 9)[i // 2 % 2]
+        want = want ^ v if i % 2 else want | v
+    assert int(r.stream("x")[3]) == want
+    assert _page_locked_mib() - before < 3
