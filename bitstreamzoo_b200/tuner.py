@@ -464,8 +464,14 @@ def precompile(srcs, candidates=None, nbits: int = 1 << 22, threads: int | None 
     ahead of timing, in parallel host threads, each with its own context
     (NVRTC runs on the host; the process-wide kernel cache then serves the
     timing runs).  Kernels do not depend on the stream length beyond its
-    word alignment, so one short run per pair (``nbits``, a multiple of 64
-    long enough for every form) compiles what every length uses.  ``only``
+    word alignment, so short runs of each pair (``nbits``, a multiple of 64
+    long enough for every form) compile what every length uses.  They repeat
+    until one compiles nothing: the second restores the first one's walk,
+    with other value names, and a segment that could not prove its
+    speculation takes its additions by look-back from then on, in kernels of
+    their own.  The inputs are borrowed device buffers as in :func:`measure`
+    (what is known of an input's bits past its length decides some folds).
+    Programs with the most source first.  ``only``
     (one set of :func:`codegen_key` values per source, or None for all)
     limits a source to the variants that will be timed.  Returns the wall
     seconds."""
@@ -481,12 +487,11 @@ def precompile(srcs, candidates=None, nbits: int = 1 << 22, threads: int | None 
         reps.setdefault(codegen_key(s), s)
     jobs = [(src, s) for i, src in enumerate(srcs) for k, s in reps.items()
             if only is None or only[i] is None or k in only[i]]
+    jobs.sort(key=lambda job: -len(job[0]))
     local = threading.local()
     ctxs = []
     lock = threading.Lock()
-    nw = (nbits + 63) // 64
-    rng = np.random.default_rng(7)
-    host_in = [rng.integers(0, 2**64, size=nw, dtype=np.uint64) for _ in range(8)]
+    bufs, inputs = _device_inputs(nbits, 8, 7)
 
     def work(job):
         if not hasattr(local, "ctx"):
@@ -498,14 +503,13 @@ def precompile(srcs, candidates=None, nbits: int = 1 << 22, threads: int | None 
         prog = local.progs.get(src)
         if prog is None:
             prog = local.progs[src] = local.ctx.compile(src)
-        r = prog.run(nbits, MODE_FUSED)
-        r.set_schedule(sched)
-        for i in range(8):
-            try:
-                r.bind(f"b{i}", host_in[i])
-            except BszError:
-                pass   # the program has fewer inputs
-        r.execute()
+        for _ in range(5):
+            r = prog.run(nbits, MODE_FUSED)
+            r.set_schedule(sched)
+            for name, (ptr, nw) in inputs.items():
+                r.bind(name, ("borrow", ptr, nw))
+            if r.execute()["compile_ms"] == 0:
+                break
 
     t0 = _time.time()
     with cf.ThreadPoolExecutor(max_workers=threads or min(16, os.cpu_count() or 4)) as ex:
@@ -514,6 +518,7 @@ def precompile(srcs, candidates=None, nbits: int = 1 << 22, threads: int | None 
                 log(f"precompiled {k + 1}/{len(jobs)} t={_time.time() - t0:.0f}s")
     for c in ctxs:
         c.close()
+    del bufs
     return _time.time() - t0
 
 
