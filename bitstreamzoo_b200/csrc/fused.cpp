@@ -1783,7 +1783,34 @@ std::unordered_map<std::string, std::shared_ptr<const SegPlan>>& plan_cache() {
 // `sc` becomes the schedule that the part takes: the register form where the
 // TMA form's argument block (a 128-byte tensor map per read input and per
 // output, 24 at most) or its boxes in one SM's shared memory would not fit.
-std::string part_source(const std::vector<Node>& nodes, const Part& p, int64_t N, Schedule& sc, PartKernel& pk) {
+// Values are named by their rank in the part, not by their number in the run's
+// graph, which differs between a program's first walk and the restored ones and
+// between trips of a loop: the same part is the same source, compiled once.
+std::string part_source(const std::vector<Node>& all, const Part& part, int64_t N, Schedule& sc, PartKernel& pk) {
+  std::vector<int> ids(part.order);
+  ids.insert(ids.end(), part.inputs.begin(), part.inputs.end());
+  for (int n : part.order)
+    for (int o : {all[n].a, all[n].b})
+      if (o >= 0) ids.push_back(o);
+  for (int n : part.outputs) ids.push_back(n);
+  for (auto& q : part.pops) ids.push_back(q.first);
+  std::sort(ids.begin(), ids.end());
+  ids.erase(std::unique(ids.begin(), ids.end()), ids.end());
+  auto rank = [&](int n) {
+    return n < 0 ? n : static_cast<int>(std::lower_bound(ids.begin(), ids.end(), n) - ids.begin());
+  };
+  std::vector<Node> nodes;
+  for (int n : ids) {
+    nodes.push_back(all[n]);
+    // an input's own operands are not in the part
+    const bool inside = std::binary_search(part.order.begin(), part.order.end(), n);
+    nodes.back().a = inside ? rank(all[n].a) : -1;
+    nodes.back().b = inside ? rank(all[n].b) : -1;
+  }
+  Part p = part;
+  for (auto* v : {&p.order, &p.inputs, &p.outputs})
+    for (int& n : *v) n = rank(n);
+  for (auto& q : p.pops) q.first = rank(q.first);
   const bool masked = (N % 64) != 0;
   if (sc.layout == 2) {
     int n_maps = static_cast<int>(p.outputs.size());

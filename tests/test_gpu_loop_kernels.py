@@ -38,3 +38,21 @@ def test_more_trips_compile_nothing_new(ctx, src, schedule):
         assert (r.int("n"), r.int("total")) == (trips, trips - 1)
         if bound is not None:
             assert r.stats["compile_ms"] == bound
+
+
+@pytest.mark.parametrize("schedule", [{"layout": 0}, {"layout": 2, "chunk_words": 4, "warps": 8, "min_blocks": 1}],
+                         ids=["warp", "tma"])
+def test_a_restored_walk_compiles_nothing_new(ctx, schedule):
+    """The second run restores the first one's walk, whose values have other
+    numbers once dead ones are left out."""
+    words = 1 << 16
+    src = ("input stream a\ninput stream b\noutput stream o\noutput int n\nstream d = a | b\nstream e = d << 9\n"
+           "stream s = a + b\nstream t = s << 2\nstream u = t ^ a\nstream g = u >> 5\no = g & s\nn = popcount(o)\n")
+    prog = ctx.compile(src)
+    rng = np.random.default_rng(4)
+    ins = {k: rng.integers(0, 2**64, words, dtype=np.uint64) for k in "ab"}
+    first = ctx.run(prog, 64 * words, ins, mode=bz.MODE_FUSED, schedule=schedule)
+    second = ctx.run(prog, 64 * words, ins, mode=bz.MODE_FUSED, schedule=schedule)
+    assert not first.stats["walk_replayed"] and second.stats["walk_replayed"]
+    assert second.stats["compile_ms"] == 0
+    assert np.array_equal(second.stream("o"), first.stream("o")) and second.int("n") == first.int("n")
