@@ -466,9 +466,8 @@ def precompile(srcs, candidates=None, nbits: int = 1 << 22, threads: int | None 
     timing runs).  Kernels do not depend on the stream length beyond its
     word alignment, so short runs of each pair (``nbits``, a multiple of 64
     long enough for every form) compile what every length uses.  They repeat
-    until one compiles nothing: the second restores the first one's walk,
-    with other value names, and a segment that could not prove its
-    speculation takes its additions by look-back from then on, in kernels of
+    until one compiles nothing and proves its speculation: a segment that
+    does not takes its additions by look-back from then on, in kernels of
     their own.  The inputs are borrowed device buffers as in :func:`measure`
     (what is known of an input's bits past its length decides some folds).
     Programs with the most source first.  ``only``
@@ -508,7 +507,8 @@ def precompile(srcs, candidates=None, nbits: int = 1 << 22, threads: int | None 
             r.set_schedule(sched)
             for name, (ptr, nw) in inputs.items():
                 r.bind(name, ("borrow", ptr, nw))
-            if r.execute()["compile_ms"] == 0:
+            st = r.execute()
+            if st["compile_ms"] == 0 and st["n_fused_fallbacks"] == 0:
                 break
 
     t0 = _time.time()
