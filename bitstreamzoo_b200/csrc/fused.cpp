@@ -2049,7 +2049,7 @@ FusedBackend::Choice FusedBackend::choose(const std::vector<Node>& nodes, const 
   };
   c.key = key();
   if (!impl_->scheduled && c.sched.layout >= 1) {
-    c.warp_next = !failed_before(threads_failed(), c.key);
+    c.warp_next = !failed_before(threads_failed(), c.key) && !failed_before(spec_failed(), c.key);
     if (!c.warp_next) {
       c.sched = Schedule{};
       c.key = key();
@@ -2386,6 +2386,7 @@ bool FusedBackend::resolve_with(const uint32_t* flags) {
   };
   size_t n = pend->parts->size(), first = unproven(flags, n);
   if (first == n) return false;
+  if (pend->nodes.empty()) throw RuntimeError("fused re-run: the graph was not kept");
   std::vector<uint32_t> warp_flags;
   std::shared_ptr<const SegPlan> warp_plan;
   if (pend->warp_next) {

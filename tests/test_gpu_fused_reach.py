@@ -63,3 +63,12 @@ def test_past_every_reach_the_result_is_exact(ctx):
     first, second = _check(ctx, SRC.replace("<< 3", "<< 29"), 70_001, 70_001, None, 2)
     assert first["n_fused_fallbacks"] >= 1
     assert second["n_fused_fallbacks"] == 0
+
+
+def test_a_schedule_that_failed_does_not_decide_for_runs_without_one(ctx):
+    """The schedule is the one that the executor picks at this length."""
+    src = SRC.replace("<< 3", "<< 31")
+    picked = {"layout": 1, "warps": 4, "min_blocks": 1, "prefetch": 0}
+    assert _check(ctx, src, 70_001, 6_000, picked, 1)[0]["n_fused_fallbacks"] >= 1
+    after = _check(ctx, src, 70_001, 6_000, None, 1)[0]
+    assert after["n_fused_fallbacks"] == 0 and after["n_fused_launches"] == 1
