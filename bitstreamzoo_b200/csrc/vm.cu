@@ -889,6 +889,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32) k_vm(const VmxArgs X) {
       if (jump >= 0) {
         if (jump >= A.n_ops) break;
         stage(jump);
+        executed += kVmStageCost;
         i = 0;
       }
     }

@@ -133,6 +133,9 @@ inline size_t vm_state_bytes(int64_t n_iregs, int64_t n_slots) {
 constexpr int64_t kVmMaxWords = 8192;
 // Instructions held in shared memory at a time.
 constexpr int kVmWindow = 1024;
+// Instructions that loading another window for a jump counts as, so that the
+// limit on executed instructions stays one on time.
+constexpr int kVmStageCost = 32;
 
 // Runs the instruction list on the context's stream as `plan` says (the plan
 // of these n_slots and nw).  `file` may be null when the file is in shared
