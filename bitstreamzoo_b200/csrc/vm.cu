@@ -383,7 +383,9 @@ __global__ void __launch_bounds__(1024) k_vm_program_loop(VmProgArgs P) {
 // Measured on a B200 (one instruction, single thread chain; the one-CTA loop
 // before it in parentheses): at 3,001 bits x ^ y 133 ns (346), x << 1 274 ns
 // (382), x + y 199 ns (742); at 400,009 bits on 16 CTAs 133 (1,458), 594
-// (1,922) and 779 ns (10,799).  A 300-op DAG of 400,009 bits: 28 us (244 us).
+// (1,922) and 779 ns (10,799).  A 300-op DAG of 400,009 bits: 28 us (244 us)
+// between device buffers, 45 us with inputs read from and results written to
+// page-locked host memory.
 constexpr int kMaxCtas = 16;      // non-portable cluster size
 constexpr int kMaxWarps = 8;      // warps per CTA
 constexpr int kMaxTotalWarps = kMaxCtas * kMaxWarps;

@@ -56,7 +56,8 @@ typedef struct bsz_stats {
   double kernel_ms;          /* CUDA-event time of the execution */
   double compile_ms;         /* time spent generating/compiling fused kernels */
   int64_t n_fused_launches;  /* generated segment kernels launched */
-  int64_t n_fused_fallbacks; /* segment parts re-run per-op because speculation was unproven */
+  int64_t n_fused_fallbacks; /* segment parts re-run per-op because speculation was unproven
+                                (a re-run in the warp form counts as a launch only) */
   int64_t n_vm_launches;     /* segments run by the device interpreter */
   int64_t walk_replayed;     /* 1: a straight-line program's statement walk was restored from
                                 the program's walk cache (same bit length, mode and bindings as
