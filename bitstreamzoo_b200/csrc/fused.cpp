@@ -1323,7 +1323,7 @@ struct GenSeq {
     if (!fn_name.empty()) {
       s << "__device__ __noinline__ void " << fn_name
         << "(const Args* __restrict__ Ap, const long long s_item, const long long e_item, const int lane) {\n"
-        // its pointers in registers (220 of 255 are taken): read from memory
+        // its pointers in registers (245 of 255 are taken): read from memory
         // again for every chunk they cost 8 % of a 512-instance batch
         << "  const Args A = *Ap;\n"
         << "  const long long L = (((e_item - s_item) + 31) / 32 + " << reg_chunk - 1 << ") / " << reg_chunk << " * "
